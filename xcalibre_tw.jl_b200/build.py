@@ -30,6 +30,9 @@ UNITS = [("xcal_kernel.cu", tag, ["-DXCAL_INST=" + tag, f"-DXCAL_NS={ns}", f"-DX
 UNITS += [("xcal_kernel.cu", "s" + tag, ["-DXCAL_INST=" + tag, f"-DXCAL_NS={ns}", f"-DXCAL_T={t}",
                                          f"-DXCAL_MB={mb}", "-DXCAL_SERVE_ONLY"])
           for tag, (ns, t, mb) in INSTANCES.items() if mb == 4 and ns >= 2]
+# the CG kernel of large meshes: Krylov value type, CTAs per SM
+UNITS += [("xcal_kernel.cu", tag, ["-DXCAL_INST=" + tag, "-DXCAL_T=" + t, "-DXCAL_MB=8", "-DXCAL_CG"])
+          for tag, t in (("cd", "double"), ("cf", "float"))]
 UNITS += [("xcal_launch.cu", None, []), ("xcal_ops.cu", None, []), ("xcal_operators.cu", None, []),
           ("xcal_api.cu", None, []),
           ("host_mesh.cpp", None, []), ("xcal_serve.cu", None, [])]

@@ -550,6 +550,15 @@ void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reord
 }
 
 // ---------------------------------------------------------- device layout
+int two_level_rows(const std::vector<int> &flev, int n, int nfl, int nbl) {
+  if (nfl != 2 || nbl != 2) return 0;
+  int n0 = 0;
+  while (n0 < n && flev[n0] == 0) ++n0;
+  for (int i = n0; i < n; ++i)
+    if (flev[i] != 1) return 0;
+  return n0;
+}
+
 int prepare(const HostMesh &M, Prep &P, std::string &err) {
   int n = (int)M.nc, nf = (int)M.nf;
   P.n = n; P.nf = nf; P.nbf = (int)M.nbf;
@@ -647,6 +656,7 @@ int prepare(const HostMesh &M, Prep &P, std::string &err) {
   }
   P.nfl = P.nbl = 1;
   for (int i = 0; i < n; ++i) { P.nfl = std::max(P.nfl, P.flev[i] + 1); P.nbl = std::max(P.nbl, P.blev[i] + 1); }
+  P.n0 = two_level_rows(P.flev, n, P.nfl, P.nbl);
   P.flev.resize(P.np, 0);
   P.blev.resize(P.np, 0);
   P.o1.resize(nf); P.o2.resize(nf);

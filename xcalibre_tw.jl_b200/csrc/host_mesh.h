@@ -50,8 +50,14 @@ struct Prep {
   std::vector<int> cb_ptr, cb_face;          // boundary faces per cell, face-id order
   std::vector<int> flev, blev;
   int nfl = 0, nbl = 0;
+  int n0 = 0;                                // two_level_rows
   std::vector<int> o1, o2;
 };
 int prepare(const HostMesh &M, Prep &P, std::string &err);
+
+// n0 > 0 when the rows [0, n0) are of level 0 and the rows [n0, n) of level 1
+// and there are no other levels in either sweep (the two-colour numbering),
+// else 0.
+int two_level_rows(const std::vector<int> &flev, int n, int nfl, int nbl);
 
 }  // namespace xcal

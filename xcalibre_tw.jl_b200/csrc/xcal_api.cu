@@ -64,6 +64,8 @@ struct xcal_ctx_s {
   int ns = 2;
   int mode = SYNC_GRID, nblocks = 1;
   int occ = 0;                 // program build: 0 = 2 CTAs/SM, 1 = 4 CTAs/SM (xcal_kernel.h)
+  CgCluster cgc{0, 0};         // pressure CG in one cluster: its form for the case (0 CTAs: not)
+  int cg_ctas = 0;             // pressure CG as a kernel on the whole GPU: its CTAs
   DevBuf mbuf, cbuf, rbuf;     // mesh, case, run buffers
   KParams hp;
   double conv = 1e-7;          // SIMPLE stop tolerance
@@ -528,7 +530,7 @@ static int mesh_prepare(xcal_ctx c, const xcal_mesh_desc *d, int32_t renumber) {
   memset(&h, 0, sizeof(h));
   const Prep &P = c->prep;
   h.n = P.n; h.nf = P.nf; h.nbf = P.nbf; h.dim = c->mesh.dim; h.ntiles = P.np / TILE;
-  h.nfl = P.nfl; h.nbl = P.nbl; h.np = P.np; h.Wf = P.Wf;
+  h.nfl = P.nfl; h.nbl = P.nbl; h.n0 = P.n0; h.np = P.np; h.Wf = P.Wf;
   return XCAL_OK;
 }
 
@@ -809,6 +811,7 @@ static int case_arrays(xcal_ctx c, const xcal_case *cfg, Sink &B, const double *
     h.Dk = A(n); h.Dw = A(n); h.Pk = A(n); h.Pw = A(n); h.G = A((size_t)n * 9);
   }
   h.done = B.zeros_n<int>(1);
+  h.step = (StepState *)B.zeros(sizeof(StepState));
   if (!B.ok()) return fail(c, B.error(), B.message());
   return XCAL_OK;
 }
@@ -836,6 +839,14 @@ int xcal_case_setup(xcal_ctx c, const xcal_case *cfg) {
     c->pin = nullptr;
     CUDA_TRY(c, stage_alloc(c, (void **)&c->pin, sizeof(double) * n * 7));
     c->pin_n = (size_t)n * 7;
+  }
+  c->cgc = CgCluster{0, 0};
+  c->cg_ctas = 0;
+  if (h.n0 > 0 && h.AP.W <= WUNROLL && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU &&
+      !(c->flags & XCAL_FLAG_CLUSTER)) {
+    const int mixed = h.prec == XCAL_PREC_MIXED;
+    c->cgc = cg_cluster(mixed, h.AP.W, h.n0, h.ntiles);
+    if (c->cgc.ctas == 0) c->cg_ctas = cg_blocks(mixed, h.AP.W, c->device);
   }
   for (bool &b : c->pin_busy) b = false;
   c->d_stage = c->cbuf.alloc<double>((size_t)n * 7);
@@ -970,6 +981,7 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   CUDA_TRY(c, cudaMemsetAsync(h.bar, 0, sizeof(Bar), c->stream));
   CUDA_TRY(c, cudaMemsetAsync(h.done, 0, sizeof(int), c->stream));
   h.mode = c->mode;
+  h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, c->occ, h.ntiles, c->nblocks);
   h.conv = c->conv;
   h.abort_nan = (c->flags & XCAL_FLAG_ABORT_ON_NAN) ? 1 : 0;
   barrier_knobs(h);
@@ -983,9 +995,27 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
     h.phase = c->d_phase;
   }
   CUDA_TRY(c, cudaEventRecord(c->ev0, c->stream));
-  if (iters > 0)
-    CUDA_TRY(c, launch_program(c->ns, h.prec == XCAL_PREC_MIXED, c->occ, c->mode, c->nblocks, &h, prog, iters,
-                               c->stream));
+  // The pressure CG over a two-level numbering as a kernel of its own between
+  // launches of the program: in one cluster where the mesh fits its shared
+  // memory, on the whole GPU where the matrix rows do not fit the CTAs' shared
+  // memory.  (Launch forms asked for by the environment keep one launch.)
+  const int mixed = h.prec == XCAL_PREC_MIXED;
+  const bool own = iters > 0 && !getenv("XCAL_NBLOCKS") && !getenv("XCAL_SYNC");
+  const CgCluster cluster = own ? c->cgc : CgCluster{0, 0};
+  const int cgb = own && cluster.ctas == 0 && c->mode == SYNC_GRID && h.ring == 0 ? std::min(c->cg_ctas, h.ntiles) : 0;
+  if (cluster.ctas > 0 || cgb > 0) {
+    CUDA_TRY(c, cudaMemsetAsync(h.step, 0, sizeof(StepState), c->stream));
+    h.ring = 0;   // the program's launches hold no matrix rows
+    const int total = iters * (prog == PROG_PISO ? 2 : 1);
+    for (int k = 0; k <= total; ++k) {
+      CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, k, c->stream));
+      if (k == total) break;
+      CUDA_TRY(c, cluster.ctas > 0 ? launch_cg_cluster(mixed, cluster, &h, c->stream)
+                                   : launch_cg(mixed, cgb, &h, c->stream));
+    }
+  } else if (iters > 0) {
+    CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, -1, c->stream));
+  }
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
   // results: one pinned block, one synchronisation
   const size_t nR = (size_t)std::max(iters, 1) * 4, nK = (size_t)std::max(iters, 1) * 5;
@@ -1259,6 +1289,7 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
   h.n = n; h.ntiles = np / TILE; h.np = np;
   TRY(upload_c(c, B, h.flev, fl)); TRY(upload_c(c, B, h.blev, bl));
   h.nfl = nfl; h.nbl = nbl;
+  h.n0 = two_level_rows(fl, n, nfl, nbl);
   TRY(upload_c(c, B, h.AU.col, ecol)); TRY(upload_c(c, B, h.AU.tpos, etp)); TRY(upload_c(c, B, h.AU.dpos, edp));
   h.AU.W = W; h.AU.np = np;
   std::vector<double> bb(b, b + n), xx(x, x + n);
@@ -1289,6 +1320,7 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
     c->ns = saved_ns; c->mode = saved_mode; c->nblocks = saved_nb; c->occ = saved_occ;
   }
   h.mode = mode;
+  h.ring = ring_tiles(W, 0, 0, h.ntiles, nb);
   if (solver == XCAL_SOLVER_GMRES) {
     double *g1 = nullptr, *g2 = nullptr;
     std::function<double *(size_t)> allocD = [&](size_t cnt) { return A(cnt); };
@@ -1297,7 +1329,7 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
   }
   CUDA_TRY(c, cudaMemsetAsync(h.bar, 0, sizeof(Bar), c->stream));
   barrier_knobs(h);
-  CUDA_TRY(c, launch_program(1, 0, 0, mode, nb, &h, PROG_SOLVE, 1, c->stream));
+  CUDA_TRY(c, launch_program(1, 0, 0, mode, nb, &h, PROG_SOLVE, 1, -1, c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   Bar bar;
   double so[2];
@@ -1735,6 +1767,7 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.conv = tolerance;
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
+  h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, gmres_ctas);   // the serving build: 4 CTAs per SM
   h.cg_fuse = 0;
   h.phase = nullptr;
   h.bar = nullptr;   // the serving loop gives the case a barrier word when it starts

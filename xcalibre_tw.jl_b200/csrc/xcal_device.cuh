@@ -35,6 +35,16 @@ struct Bar {
   unsigned long long count;
   int err;
   int nonfinite;   // set when a run stopped on a non-finite residual
+  unsigned exits;  // CTAs that left a launch which another one follows
+  unsigned pad;
+};
+
+// What the launches of a run that is cut at its pressure solves hand on.
+struct StepState {
+  int finite, stop;   // Krylov norms of the iteration finite so far; the run has ended
+  int pw;             // partial-sum buffer the next reduction writes
+  int its;            // the solve: iterations, residual norm
+  double rnorm;
 };
 
 struct BcEntry {
@@ -68,6 +78,12 @@ struct MatT {
 };
 using Mat = MatT<double>;
 
+// CG in one cluster (xcal_cg_cluster_kernel): threads and vectors per CTA,
+// most tiles of the mesh (one partial per lane of the final sum) and of a CTA.
+constexpr int CGC_TPB = 1024, CGC_VECTORS = 8, CGC_TILES = 256, CGC_SLOTS = 16;
+// Tiles of a group (count N) given to CTA b of G: [chunk(b), chunk(b+1)).
+__host__ __device__ inline int chunk(int b, int N, int G) { return (int)((long long)b * N / G); }
+
 struct KCfg {
   int solver, itmax;
   double atol, rtol;
@@ -100,6 +116,8 @@ struct KParams {
   const int *cb_ptr, *cb_face;
   const int *flev, *blev;                 // [np]
   int nfl, nbl;
+  int n0;          // rows [0, n0) of DILU level 0 and [n0, n) of level 1, all of them (0: any other numbering)
+  int ring;        // matrix tiles the launch's dynamic shared memory holds (row width W, the Krylov value type)
   int cg_fuse;     // CG: M^{-1} of a two-level DILU inside the x/r phase (2 barriers per iteration)
   int abort_nan;   // stop at the first non-finite Krylov residual norm
   double conv;     // SIMPLE stop: every residual <= conv (1e-7 in the reference)
@@ -133,6 +151,7 @@ struct KParams {
   int *kry;             // [iters * 5]
   int *done;            // iterations executed
   Bar *bar;
+  StepState *step;
   // standalone solve
   double *sb;
   int solve_solver, solve_itmax;
@@ -252,9 +271,9 @@ struct Sync {
   unsigned extra;                  // arrivals expected beyond the nb CTAs (0)
   unsigned long long timeout_ns;   // limit of one wait
   unsigned long long epoch;
-  int *ok;   // shared flag
 
-  __device__ __forceinline__ bool sync() {
+  // s_ok: a flag in shared memory
+  __device__ __forceinline__ bool sync(int *s_ok) {
     if (mode == SYNC_BLOCK) { __syncthreads(); return true; }
     if (mode == SYNC_CLUSTER) {
       __syncthreads();
@@ -284,10 +303,10 @@ struct Sync {
       }
       // the acquire (poll, or the arrive of the last CTA) orders the CTA's
       // later loads, through the block barrier below, after every arrive
-      *ok = good;
+      *s_ok = good;
     }
     __syncthreads();
-    return *ok != 0;
+    return *s_ok != 0;
   }
 };
 
@@ -333,7 +352,16 @@ __device__ __forceinline__ void final_sum(const double *part, int ntiles, double
     const double *pp = part + (size_t)k * ntiles;
     const int t = threadIdx.x;
     double a = (t < ntiles) ? pp[t] : 0.0;
-    for (int q = t + TPB; q < ntiles; q += TPB) a = a + pp[q];
+    // ascending, eight loads in flight at a time
+    int q = t + TPB;
+    for (; q + 7 * TPB < ntiles; q += 8 * TPB) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = pp[q + u * TPB];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a = a + v[u];
+    }
+    for (; q < ntiles; q += TPB) a = a + pp[q];
     s[k] = a;
   }
 #pragma unroll

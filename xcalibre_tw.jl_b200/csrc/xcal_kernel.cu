@@ -19,6 +19,15 @@ namespace {
 __shared__ int s_vbid, s_vnb;
 __device__ __forceinline__ int vbid() { return s_vbid; }
 __device__ __forceinline__ int vnb() { return s_vnb; }
+// Scratch of the reductions and the phase timers.  File scope, so that the
+// out-of-line solvers address them as shared memory and not through generic
+// pointers.
+constexpr int MAXTL = 8;                 // tiles per CTA whose warp sums are staged
+__shared__ double s_sm[8 * MAXK];
+__shared__ double s_out[MAXK];
+__shared__ double s_ws[MAXTL * MAXK * 8];
+__shared__ int s_ok;
+__shared__ unsigned long long s_pacc[2 * NPH];   // per-phase cycles and counts
 
 
 // Level-scheduled preconditioners (forward and backward sweeps): DILU, ILU(0).
@@ -47,10 +56,15 @@ __device__ __forceinline__ void lev_bwd_row(const MatT<T> &A, const T *out, int 
   else dilu_bwd_row_g<NS>(A, oi, g, i, o);
 }
 
-constexpr int MAXTL = 32;   // tiles per CTA whose warp sums are staged in shared memory
-
+// State of the CTA's run.  The mesh scalars the solvers use are copied here
+// from KParams: a solver called out of line takes a copy of the whole struct
+// into registers instead of reaching through a pointer for each of them.
 struct Ctx {
   const KParams *P;
+  int n, np, ntiles, nfl, nbl, cg_fuse;
+  int n0, ring;   // rows of level 0 of a two-level numbering (0: other numberings); matrix tiles the dynamic shared memory holds
+  const int *flev, *blev;
+  int copies;     // rounds of bulk copies done (the parity of their barrier)
   Sync S;
   // Per-tile partial sums, two buffers of MAXK*ntiles used in turn by
   // successive reducing phases.  A CTA reads a reduction's partials after the
@@ -60,35 +74,60 @@ struct Ctx {
   // phases later, behind a barrier every CTA reaches only after its read.
   double *part;
   int pw;   // buffer the next reducing phase writes
-  __device__ __forceinline__ double *part_w() const { return part + (size_t)pw * MAXK * P->ntiles; }
-  __device__ __forceinline__ const double *part_r() const { return part + (size_t)(pw ^ 1) * MAXK * P->ntiles; }
-  double *sm;       // [8*MAXK]
-  double *sm_out;   // [MAXK]
-  double *ws;       // [MAXTL*MAXK*8] staged warp sums
+  __device__ __forceinline__ double *part_w() const { return part + (size_t)pw * MAXK * ntiles; }
+  __device__ __forceinline__ const double *part_r() const { return part + (size_t)(pw ^ 1) * MAXK * ntiles; }
   // per-phase timers: thread 0 of CTA 0 charges the SM cycles between two
   // barrier exits to the phase class that was current at the second one
   bool timers;
   int tag;
   long long t_last;
-  unsigned long long *pacc;   // shared [2*NPH]: cycles, counts
   // Traversal direction of the tile loops, reversed at every barrier: a phase
   // then starts on the tiles the previous phase touched last, whose data are
   // the most likely still in L2 when the working set is larger than L2.  Every
   // row's values are independent of the order, so results are unchanged.
   int rev;
   __device__ __forceinline__ void phase(int t) { tag = t; }
-  __device__ __forceinline__ bool sync() {
-    rev ^= 1;
-    const bool ok = S.sync();
+  __device__ __forceinline__ void tick() {
     if (timers) {
       const long long t = clock64();
-      pacc[tag] += (unsigned long long)(t - t_last);
-      pacc[NPH + tag] += 1ull;
+      s_pacc[tag] += (unsigned long long)(t - t_last);
+      s_pacc[NPH + tag] += 1ull;
       t_last = t;
     }
+  }
+  // One value per tile summed over all tiles: put_part of every own tile
+  // (over one or more phases), then end_sum, which is a barrier of the whole
+  // group and gives every thread the canonical sum.
+  __device__ __forceinline__ void put_part(int t, double v) { part_w()[t] = v; }
+  __device__ __forceinline__ bool end_sum(double &out, bool ok) {
+    if (!ok) atomicExch(&S.bar->err, ST_TIMEOUT);   // the barrier then ends for every CTA
+    pw ^= 1;
+    if (!sync()) return false;
+    double r[1];
+    final_sum<1>(part_r(), ntiles, s_sm, s_out, r);
+    out = r[0];
+    return true;
+  }
+  __device__ __forceinline__ bool sync() {
+    rev ^= 1;
+    const bool ok = S.sync(&s_ok);
+    tick();
     return ok;
   }
 };
+
+__device__ __forceinline__ void ctx_mesh(Ctx &C, const KParams &P) {
+  C.P = &P;
+  C.n = P.n;
+  C.np = P.np;
+  C.ntiles = P.ntiles;
+  C.nfl = P.nfl;
+  C.nbl = P.nbl;
+  C.cg_fuse = P.cg_fuse;
+  C.n0 = P.n0;
+  C.ring = P.ring;
+  C.copies = 0;
+}
 
 template <typename T>
 __device__ __forceinline__ const MatT<T> &matU(const KParams &P) {
@@ -120,7 +159,7 @@ __device__ __forceinline__ int own_tile(int m, int cnt, int rev) {
 
 template <class F>
 __device__ __forceinline__ void tile_each(const Ctx &C, F f) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const int cnt = own_tiles(P.ntiles);
   for (int m = 0; m < cnt; ++m) {
     const int i = own_tile(m, cnt, C.rev) * TILE + threadIdx.x;
@@ -136,7 +175,7 @@ __device__ __forceinline__ void tile_each(const Ctx &C, F f) {
 // warps are not held at a block barrier per tile.
 template <int K, class F>
 __device__ __forceinline__ void tile_phase(Ctx &C, bool reduce, F f) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const int nt = P.ntiles, cnt = own_tiles(nt), rev = C.rev;
   if (!reduce) {
     for (int m = 0; m < cnt; ++m) {
@@ -161,12 +200,12 @@ __device__ __forceinline__ void tile_phase(Ctx &C, bool reduce, F f) {
       for (int k = 0; k < K; ++k) {
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) v[k] = v[k] + __shfl_down_sync(0xffffffffu, v[k], off);
-        if (lane == 0) C.ws[(tl * K + k) * 8 + wid] = v[k];
+        if (lane == 0) s_ws[(tl * K + k) * 8 + wid] = v[k];
       }
     }
     __syncthreads();
     for (int q = threadIdx.x; q < tn * K; q += TPB) {
-      const double *w = C.ws + q * 8;
+      const double *w = s_ws + q * 8;
       double a0 = w[0] + w[4], a1 = w[1] + w[5];
       const double a2 = w[2] + w[6], a3 = w[3] + w[7];
       a0 = a0 + a2;
@@ -191,7 +230,7 @@ struct CgRows {
 // Row pairs pay when the CTAs hold two tiles or more each; with one tile per
 // CTA or fewer (small meshes: one phase is a barrier and one row per thread)
 // the one-row routines are faster.  Uniform across the CTAs of a run.
-__device__ __forceinline__ bool pairs_pay(const KParams &P) { return P.ntiles >= 2 * vnb(); }
+__device__ __forceinline__ bool pairs_pay(const Ctx &P) { return P.ntiles >= 2 * vnb(); }
 
 // tile_phase over R tiles at a time: the CTA takes its tiles (in the phase's
 // direction) R by R, thread t row t of each (ii[r], ok[r] false past the
@@ -199,7 +238,7 @@ __device__ __forceinline__ bool pairs_pay(const KParams &P) { return P.ntiles >=
 // those of tile_phase (each tile's canonical tree).
 template <int K, int R, class F>
 __device__ __forceinline__ void tile_phase_rows(Ctx &C, bool reduce, F f) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const int nt = P.ntiles, cnt = own_tiles(nt), rev = C.rev;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double *part = C.part_w();
@@ -231,14 +270,14 @@ __device__ __forceinline__ void tile_phase_rows(Ctx &C, bool reduce, F f) {
             double x = v[r][k];
 #pragma unroll
             for (int off = 16; off >= 1; off >>= 1) x = x + __shfl_down_sync(0xffffffffu, x, off);
-            if (lane == 0) C.ws[((tl + r) * K + k) * 8 + wid] = x;
+            if (lane == 0) s_ws[((tl + r) * K + k) * 8 + wid] = x;
           }
         }
     }
     if (!reduce) continue;
     __syncthreads();
     for (int q = threadIdx.x; q < tn * K; q += TPB) {
-      const double *w = C.ws + q * 8;
+      const double *w = s_ws + q * 8;
       double a0 = w[0] + w[4], a1 = w[1] + w[5];
       const double a2 = w[2] + w[6], a3 = w[3] + w[7];
       a0 = a0 + a2;
@@ -271,8 +310,8 @@ __device__ __forceinline__ void st(double *a, int i, const double (&o)[NS]) {
 // Row-local part of M^{-1}: DILU forward level 0 (and the backward step of
 // rows without upper neighbours) or a diagonal scaling.  Returns false when
 // the row has no row-local part (DILU rows of level >= 1).
-template <int NS, typename T>
-__device__ __forceinline__ bool precon_local(const KParams &P, const MatT<T> &A, int i, const T (&in)[NS],
+template <int NS, typename T, class PT>
+__device__ __forceinline__ bool precon_local(const PT &P, const MatT<T> &A, int i, const T (&in)[NS],
                                              T (&o)[NS]) {
   if (A.precon == PRECON_DILU) {
     if (ldro(P.flev + i) != 0) return false;
@@ -305,7 +344,7 @@ __device__ __forceinline__ bool precon_local(const KParams &P, const MatT<T> &A,
 // Number of phases of M^{-1} after its producer phase.  The producer did the
 // row-local part (and, with first_lvl == 2, forward level 1 as well).
 template <typename T>
-__device__ __forceinline__ int precon_tail_phases(const KParams &P, const MatT<T> &A, bool setup, int first_lvl) {
+__device__ __forceinline__ int precon_tail_phases(const Ctx &P, const MatT<T> &A, bool setup, int first_lvl) {
   if (!leveled(A)) return setup ? 1 : 0;
   return max(0, P.nfl - first_lvl) + (P.nbl - 1);
 }
@@ -315,7 +354,7 @@ __device__ __forceinline__ int precon_tail_phases(const KParams &P, const MatT<T
 // The last phase also computes the K partial sums red(i, v).
 template <int NS, int K, typename T, class Red, int R = 1>
 __device__ __forceinline__ bool precon_tail(Ctx &C, const MatT<T> &A, const T *in, T *out, bool setup, int first_lvl, Red red) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const int nph = precon_tail_phases(P, A, setup, first_lvl);
   C.phase(setup ? PH_PREC_SETUP : PH_KRY_PREC);
   if constexpr (R > 1) {
@@ -512,9 +551,9 @@ __device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWo
 template <int NS, typename T>
 __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *bb, const KCfg &cfg,
                          int (&its)[NS], double (&rnorm_out)[NS]) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   double red[2 * NS];
-  final_sum<2 * NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+  final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
   double rho[NS], alpha[NS], omega[NS], beta[NS], rnorm[NS], eps[NS], nrho[NS];
   unsigned active = 0;
 #pragma unroll
@@ -572,7 +611,7 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
       return false;
     {
       double cv[NS];
-      final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, cv);
+      final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, cv);
 #pragma unroll
       for (int d = 0; d < NS; ++d)
         if (active & (1u << d)) alpha[d] = rho[d] / cv[d];
@@ -618,7 +657,7 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
           }
         }))
       return false;
-    final_sum<2 * NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+    final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
 #pragma unroll
     for (int d = 0; d < NS; ++d)
       if (active & (1u << d)) omega[d] = red[2 * d] / red[2 * d + 1];
@@ -640,7 +679,7 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
       }
     });
     if (!C.sync()) return false;
-    final_sum<2 * NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+    final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
     unsigned cont = 0;
 #pragma unroll
     for (int d = 0; d < NS; ++d) {
@@ -663,6 +702,289 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
   return true;
 }
 
+// ------------------------------------------- CG over a two-level numbering
+// The two-colour numbering (quad and hex meshes) puts the rows of DILU level
+// 0 first: rows [0, n0) have only upper neighbours, rows [n0, n) only lower
+// ones.  CG then needs no level arrays, and its phases touch only the rows
+// they change (the arithmetic of each row is that of cg() below):
+//   A  all rows: p = z + beta p, q = A p, <p, q>; x += alpha p of the
+//      iteration before (its p is read here in any case)
+//   B  level 1: r -= alpha q, z = M^-1 r (neighbours' r recomputed)
+//   C  level 0: r -= alpha q, z = M^-1 r; <r, z>
+// A tile's <r, z> is summed in the phase that completes it.
+//
+// RES: the CTA's matrix tiles (values and columns) are copied into shared
+// memory at the start of the solve by bulk copies of one thread (the 256
+// entries of one row position are contiguous in the ELL layout) and stay
+// there: after a barrier, which empties L1, the columns come from shared
+// memory at once and the phase is one round of gathers long instead of two.
+// Otherwise the rows are read from global memory in every phase.
+extern __shared__ __align__(128) unsigned char s_dyn[];
+__shared__ unsigned long long s_full;   // mbarrier: the matrix tiles have arrived
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned long long *b, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_inval(unsigned long long *b) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned long long *b, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(b)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Waits for the phase of the given parity, at most limit_ns.
+__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, unsigned long long limit_ns) {
+  if (mbar_try(b, parity)) return true;
+  const unsigned long long t = globaltimer();
+  while (!mbar_try(b, parity))
+    if (globaltimer() - t > limit_ns) return false;
+  return true;
+}
+// Copy of `bytes` (a multiple of 16; both addresses 16-byte aligned) into shared memory.
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, unsigned long long *b) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(b))
+               : "memory");
+}
+
+// The barrier of the copies, by the whole CTA at the start of a launch or of
+// a serving job (`again`: the barrier of the job before is given up).
+__device__ __forceinline__ void copies_init(bool again) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (again) mbar_inval(&s_full);
+    mbar_init(&s_full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+}
+
+template <typename T, int WT, bool RES>
+__device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int &its_out,
+                                             double &rn_out) {
+  constexpr double EPS = 2.220446049250313e-16;
+  constexpr int CAP = MAXTL * MAXK;   // tiles whose warp sums fit s_ws
+  const int n = C.n, n0 = C.n0, np = A.np, nt = C.ntiles;
+  const int W = WT < WUNROLL ? WT : A.W;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int B0 = vbid(), G = vnb();
+  const int cnt = own_tiles(nt);
+  const int t0 = (n0 - 1) / TILE, t1 = n0 / TILE;        // last tile with level-0 rows, first with level-1 rows
+  const int c0 = own_tiles(t0 + 1);                      // own tiles with level-0 rows: m in [0, c0)
+  const int m1 = t1 > B0 ? min(cnt, (t1 - B0 + G - 1) / G) : 0;   // with level-1 rows: m in [m1, cnt)
+  T *sv = (T *)s_dyn;
+  int *sc = (int *)(s_dyn + (size_t)C.ring * W * TILE * sizeof(T));
+  bool arrived = true;
+  if (RES) {
+    if (tid == 0) {
+      // the matrix was written through ordinary stores, which this thread has
+      // acquired with the last barrier: order them before the bulk copies
+      asm volatile("fence.proxy.async;" ::: "memory");
+      mbar_expect(&s_full, cnt * W * TILE * (unsigned)(sizeof(T) + sizeof(int)));
+      for (int m = 0; m < cnt; ++m)
+        for (int k = 0; k < W; ++k) {
+          const size_t e = (size_t)k * np + (size_t)(B0 + G * m) * TILE;
+          bulk_copy(sv + (size_t)(m * W + k) * TILE, A.val + e, TILE * sizeof(T), &s_full);
+          bulk_copy(sc + (size_t)(m * W + k) * TILE, A.col + e, TILE * sizeof(int), &s_full);
+        }
+    }
+    arrived = mbar_wait(&s_full, C.copies & 1, C.S.timeout_ns);
+    C.copies += 1;
+  }
+  // first entry of row i of own tile m; entry k is at [k * ks]
+  const size_t ks = RES ? (size_t)TILE : (size_t)np;
+  auto vals = [&](int m) -> const T * {
+    return RES ? sv + (size_t)m * W * TILE + tid : A.val + (size_t)(B0 + G * m) * TILE + tid;
+  };
+  auto cols = [&](int m) -> const int * {
+    return RES ? sc + (size_t)m * W * TILE + tid : A.col + (size_t)(B0 + G * m) * TILE + tid;
+  };
+  // warp sum of a tile's products into s_ws[q]; block sums of the staged own
+  // tiles m0, m0+d, ... to the partials
+  auto stage = [&](int q, double v) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) s_ws[q * 8 + wid] = v;
+  };
+  auto tile_sums = [&](int m0, int d, int count) {
+    __syncthreads();
+    if (tid < count) {
+      const double *ww = s_ws + tid * 8;
+      double a0 = ww[0] + ww[4], a1 = ww[1] + ww[5];
+      const double a2 = ww[2] + ww[6], a3 = ww[3] + ww[7];
+      a0 = a0 + a2;
+      a1 = a1 + a3;
+      C.put_part(B0 + G * (m0 + d * tid), a0 + a1);
+    }
+  };
+
+  double red[1];
+  final_sum<1>(C.part_r(), nt, s_sm, s_out, red);
+  const double sgn = (red[0] < 0.0) ? -1.0 : 1.0;
+  double gamma = sgn * red[0], rnorm = sqrt(gamma), alpha = 0.0, beta = 0.0, pn2 = gamma;
+  int its = 0;
+  bool active = false;
+  double eps = 0.0;
+  if (gamma != 0.0) {
+    eps = cfg.atol + cfg.rtol * rnorm;
+    active = !(rnorm <= eps || 0 >= cfg.itmax);
+  }
+  T *z = w.v[0];
+  T *ro = w.r[0], *rn = w.r[1], *pn = w.p[0], *pspare = w.p[1];
+  // The first direction is z itself: z + beta z and x + alpha z with beta =
+  // alpha = 0 (exact for finite z; a non-finite z makes gamma, and with it
+  // alpha and the result, non-finite), so the row loop has no branch that
+  // would keep its loads from being issued together.
+  const T *po = z;
+  bool pending = false;   // x still lacks alpha*po
+  while (active) {
+    // A
+    C.phase(PH_KRY_SPMV);
+    for (int m = 0, q = 0; m < cnt; ++m) {
+      const int i = (B0 + G * m) * TILE + tid;
+      const T *v = vals(m);
+      const int *c = cols(m);
+      double pq = 0.0;
+      if (i < n) {
+        const T xi = w.x[i];
+        T y = T(0), pi = T(0), poi = T(0);
+#pragma unroll
+        for (int k = 0; k < WT; ++k) {
+          const int kk = (WT < WUNROLL || k < W) ? k : W - 1;
+          const int cj = (WT < WUNROLL || k < W) ? c[kk * ks] : -1;
+          const int j = cj >= 0 ? cj : i;
+          const T oj = po[j], pj = vaxpy<T>(z[j], beta, oj);
+          const T t = y + v[kk * ks] * pj;
+          y = cj >= 0 ? t : y;
+          if (cj == i) {
+            pi = pj;
+            poi = oj;
+          }
+        }
+        w.x[i] = vaxpy<T>(xi, alpha, poi);
+        pn[i] = pi;
+        w.q[i] = y;
+        pq = (double)pi * (double)y;
+      }
+      stage(q, pq);
+      if (++q == CAP || m + 1 == cnt) {
+        tile_sums(m + 1 - q, 1, q);
+        q = 0;
+        if (m + 1 < cnt) __syncthreads();
+      }
+    }
+    pending = false;
+    double s;
+    if (!C.end_sum(s, arrived)) return false;
+    const double pAp = sgn * s;
+    if (pAp <= EPS * pn2 && fabs(pAp) <= EPS * pn2) break;   // zero curvature: stop
+    alpha = gamma / pAp;
+    // B
+    C.phase(PH_KRY_PREC);
+    for (int m = cnt - 1, q = 0; m >= m1; --m) {
+      const int i = (B0 + G * m) * TILE + tid;
+      const T *v = vals(m);
+      const int *c = cols(m);
+      double rz = 0.0;
+      if (i < n && i >= n0) {
+        const T ri = vaxpy<T>(ro[i], -alpha, w.q[i]), di = A.Dinv[i];
+        T o = ri;
+#pragma unroll
+        for (int k = 0; k < WT - 1; ++k) {   // the diagonal is the last entry
+          const int kk = (WT < WUNROLL || k < W - 1) ? k : 0;
+          const int cj = (WT < WUNROLL || k < W - 1) ? c[kk * ks] : -1;
+          const bool use = cj >= 0 && cj < i;
+          const int j = use ? cj : i;
+          const T t = o - v[kk * ks] * vaxpy<T>(ro[j], -alpha, w.q[j]) * A.Dinv[j];
+          o = use ? t : o;
+        }
+        o = o * di;
+        rn[i] = ri;
+        z[i] = o;
+        rz = (double)ri * (double)o;
+      }
+      if (m >= c0) {   // no level-0 rows: the tile is complete
+        stage(q, rz);
+        if (++q == CAP || m == max(m1, c0)) {
+          tile_sums(m + q - 1, -1, q);
+          q = 0;
+          __syncthreads();
+        }
+      }
+    }
+    if (!C.sync()) return false;
+    // C
+    C.phase(PH_KRY_PREC);
+    for (int m = c0 - 1, q = 0; m >= 0; --m) {
+      const int i = (B0 + G * m) * TILE + tid;
+      const T *v = vals(m);
+      const int *c = cols(m);
+      double rz = 0.0;
+      if (i < n0) {
+        const T ri = vaxpy<T>(ro[i], -alpha, w.q[i]);
+        const T di = A.Dinv[i];
+        T o = ri * di;
+#pragma unroll
+        for (int k = 1; k < WT; ++k) {   // the diagonal is the first entry
+          const int kk = (WT < WUNROLL || k < W) ? k : W - 1;
+          const int cj = (WT < WUNROLL || k < W) ? c[kk * ks] : -1;
+          const bool use = cj > i;
+          const int j = use ? cj : i;
+          const T t = o - v[kk * ks] * z[j] * di;
+          o = use ? t : o;
+        }
+        rn[i] = ri;
+        z[i] = o;
+        rz = (double)ri * (double)o;
+      } else if (i < n) {   // level-1 rows of the tile that holds both levels
+        rz = (double)rn[i] * (double)z[i];
+      }
+      stage(q, rz);
+      if (++q == CAP || m == 0) {
+        tile_sums(m + q - 1, -1, q);
+        q = 0;
+        if (m > 0) __syncthreads();
+      }
+    }
+    if (!C.end_sum(s, arrived)) return false;
+    const double gn = sgn * s;
+    rnorm = sqrt(gn);
+    const bool solved = (rnorm <= eps) || (rnorm + 1.0 <= 1.0);
+    if (!solved) {
+      beta = gn / gamma;
+      pn2 = gn + (beta * beta) * pn2;
+      gamma = gn;
+    }
+    its += 1;
+    active = !(solved || its >= cfg.itmax);
+    pending = true;
+    T *tp = ro;
+    ro = rn;
+    rn = tp;
+    tp = pn;
+    pn = pspare;
+    pspare = tp;
+    po = tp;
+  }
+  if (pending)   // x += alpha p of the last iteration: own rows, read by this thread only before the next barrier
+    for (int m = 0; m < cnt; ++m) {
+      const int i = (B0 + G * m) * TILE + tid;
+      if (i < n) w.x[i] = vaxpy<T>(w.x[i], alpha, po[i]);
+    }
+  its_out = its;
+  rn_out = rnorm;
+  return true;
+}
+
 // ------------------------------------------------------------------- CG
 // Krylov.jl 0.9.5 cg! with preconditioner M.  The sign of <r,z> at the start
 // selects the formulation: for a negative definite system CG runs on (-A)x=-b,
@@ -676,10 +998,10 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
 template <int NS, typename T>
 __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                    double (&rnorm_out)[NS]) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const double EPS = 2.220446049250313e-16;
   double red[NS];
-  final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+  final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
   double gamma[NS], sgn[NS], rnorm[NS], pn2[NS], eps[NS], alpha[NS], beta[NS];
   unsigned active = 0;
 #pragma unroll
@@ -748,7 +1070,7 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
       });
     }
     if (!C.sync()) return false;
-    final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+    final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
     unsigned upd = 0;
 #pragma unroll
     for (int d = 0; d < NS; ++d) {
@@ -877,7 +1199,7 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
       };
       if (!precon_tail<NS, NS, T, decltype(rz), CgRows<T>::R>(C, A, (const T *)rn, zw, false, 2, rz)) return false;
     }
-    final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+    final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
     unsigned cont = 0;
 #pragma unroll
     for (int d = 0; d < NS; ++d) {
@@ -946,10 +1268,10 @@ __device__ __forceinline__ void sym_givens(double a, double b, double &c, double
 template <int NS, typename T>
 __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                       double (&rnorm_out)[NS]) {
-  const KParams &P = *C.P;
+  const Ctx &P = C;
   const double BTOL = 1.8189894035458565e-12;   // eps(Float64)^(3/4) = 2^-39
   double red[2 * NS];
-  final_sum<2 * NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
+  final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
   const int G1 = w.gmax + 1;
   const int kmax = min(cfg.itmax, w.gmax);
   double *gws = w.gws + (size_t)vbid() * NS * 4 * G1;
@@ -1015,7 +1337,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
         }))
       return false;
     double h[NS];
-    final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, h);
+    final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, h);
     if (threadIdx.x == 0)
 #pragma unroll
       for (int d = 0; d < NS; ++d) gws[(size_t)d * 4 * G1 + 3 * G1] = h[d];
@@ -1035,7 +1357,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
         }
       });
       if (!C.sync()) return false;
-      final_sum<NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, h);
+      final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, h);
       if (!norm && threadIdx.x == 0)
 #pragma unroll
         for (int d = 0; d < NS; ++d) gws[(size_t)d * 4 * G1 + 3 * G1 + (m - 1)] = h[d];
@@ -1061,7 +1383,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
         const double zeta = s_ * zz[k - 1];
         zz[k - 1] = c_ * zz[k - 1];
         zz[k] = zeta;
-        C.sm_out[d] = fabs(zeta);
+        s_out[d] = fabs(zeta);
         if (vbid() == 0) {
           double *Rc = w.gR + (size_t)d * rs + (size_t)(k - 1) * k / 2;
           for (int i = 0; i < k; ++i) Rc[i] = col[i];
@@ -1073,7 +1395,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
 #pragma unroll
     for (int d = 0; d < NS; ++d) {
       if (!(active & (1u << d))) continue;
-      rnorm[d] = C.sm_out[d];
+      rnorm[d] = s_out[d];
       its[d] = k;
       const bool mach = (rnorm[d] + 1.0 <= 1.0);
       const bool solved = (rnorm[d] <= eps[d]) || mach;
@@ -1123,12 +1445,75 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
   return true;
 }
 
+// The general solvers out of line, once per component count: inlined at each
+// call they made the program several times larger and its build minutes
+// longer.  The state and the operands are copied in (and the state back), so
+// the caller's own state stays in registers and the solver works on registers.
+template <int NS, typename T>
+__device__ __noinline__ bool krylov_general(Ctx *state, MatT<T> A, KWorkT<T> w, const double *b, KCfg cfg, int *its,
+                                            double *rn) {
+  Ctx C = *state;
+  int it[NS];
+  double r[NS];
+  bool ok;
+  if (cfg.solver == SOLVER_BICGSTAB) ok = bicgstab<NS, T>(C, A, w, b, cfg, it, r);
+  else if (cfg.solver == SOLVER_GMRES) ok = gmres<NS, T>(C, A, w, cfg, it, r);
+  else ok = cg<NS, T>(C, A, w, cfg, it, r);
+#pragma unroll
+  for (int d = 0; d < NS; ++d) {
+    its[d] = it[d];
+    rn[d] = r[d];
+  }
+  *state = C;
+  return ok;
+}
 template <int NS, typename T>
 __device__ __forceinline__ bool krylov(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, const KCfg &cfg,
-                       int solver, int (&its)[NS], double (&rn)[NS]) {
-  if (solver == SOLVER_BICGSTAB) return bicgstab<NS, T>(C, A, w, b, cfg, its, rn);
-  if (solver == SOLVER_GMRES) return gmres<NS, T>(C, A, w, cfg, its, rn);
-  return cg<NS, T>(C, A, w, cfg, its, rn);
+                                       int (&its)[NS], double (&rn)[NS]) {
+  Ctx t = C;
+  int it[NS];
+  double r[NS];
+  const bool ok = krylov_general<NS, T>(&t, A, w, b, cfg, it, r);
+#pragma unroll
+  for (int d = 0; d < NS; ++d) {
+    its[d] = it[d];
+    rn[d] = r[d];
+  }
+  C = t;
+  return ok;
+}
+
+// Momentum solve: BiCGSTAB with DILU, the configurations' solver, inlined
+// (its operands are then the kernel's parameters).
+template <int NS, typename T>
+__device__ __forceinline__ bool solve_vector(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
+                                             const KCfg &cfg, int (&its)[NS], double (&rn)[NS]) {
+  if (cfg.solver == SOLVER_BICGSTAB && A.precon == PRECON_DILU) return bicgstab<NS, T>(C, A, w, b, cfg, its, rn);
+  return krylov<NS, T>(C, A, w, b, cfg, its, rn);
+}
+
+// Scalar solve of a mesh of DIM dimensions: the two-level CG inlined here,
+// where its operands are the kernel's parameters, the general solvers out of
+// line.
+template <int DIM, typename T>
+__device__ __forceinline__ bool solve_scalar(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
+                                             const KCfg &cfg, int (&its)[1], double (&rn)[1]) {
+  constexpr int WT = DIM == 2 ? 5 : DIM == 3 ? 7 : WUNROLL;   // rows of a quad or hex mesh
+  if (cfg.solver == SOLVER_CG && A.precon == PRECON_DILU && C.n0 > 0 && A.W <= WUNROLL) {
+    // (large meshes run the CG as a kernel of its own; here the rows of tiles
+    // that do not fit are those of a standalone solve or of a serving case)
+    if (C.ring * vnb() < C.ntiles) {
+#if defined(XCAL_SERVE_ONLY)
+      if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, false>(C, A, w, cfg, its[0], rn[0]);
+#endif
+      return cg_two_level<T, WUNROLL, false>(C, A, w, cfg, its[0], rn[0]);
+    }
+    if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, true>(C, A, w, cfg, its[0], rn[0]);
+    return cg_two_level<T, WUNROLL, true>(C, A, w, cfg, its[0], rn[0]);
+  }
+  if (DIM == 2 && cfg.solver == SOLVER_BICGSTAB && A.precon == PRECON_DILU)   // k and omega
+    return bicgstab<1, T>(C, A, w, b, cfg, its, rn);
+  return krylov<1, T>(C, A, w, b, cfg, its, rn);
 }
 
 // -------------------------------------------------------------- assembly
@@ -1627,7 +2012,7 @@ __device__ __forceinline__ bool turbulence(Ctx &C) {
     if (!krylov_start<1, T>(C, A, wk, P.bP, cfg.solver)) return false;
     int its[1];
     double rn[1];
-    if (!krylov<1, T>(C, A, wk, P.bP, cfg, cfg.solver, its, rn)) return false;
+    if (!solve_scalar<NS, T>(C, A, wk, P.bP, cfg, its, rn)) return false;
     // run! copy-back, then constrain_boundary! for omega (:401-448)
     C.phase(PH_TURB);
     tile_each(C, [&](int i) {
@@ -1674,180 +2059,230 @@ __device__ __forceinline__ bool turbulence(Ctx &C) {
 }
 
 // ------------------------------------------------------------- programs
+// A run is a chain of steps, one pressure solve each: step k = it*ncorr +
+// corr.  before_solve does everything between two solves up to the start of
+// solve k, after_solve everything that follows solve k-1 up to the end of its
+// corrector and, with the last corrector, of its iteration.
 template <int NS, typename T>
-__device__ __forceinline__ void simple_program(Ctx &C, int iters, bool piso) {
-  const KParams &P = *C.P;
-  const bool mid = (P.grad == GRAD_MIDPOINT);
-  const double nu = P.nu;
+struct Simple {
+  Ctx &C;
+  const bool piso;
+  const int ncorr;
+  bool finite;   // Krylov residual norms of this iteration all finite
+
   // set-up before the loop (Solvers_1_SIMPLE.jl:114-119)
-  C.phase(PH_SETUP);
-  grid_each(P.nf, [&](int f) {
-    face_mdot<NS>(P, f);
-    P.pf[f] = face_scalar(P, P.p, f, P.bcP, mid);
-    if (P.model == 1) P.nutf[f] = 0.0;   // initialise_RANS: a fresh face field
-    P.nueff[f] = (P.model == 1) ? nu + 0.0 : nu;
-  });
-  if (!C.sync()) return;
-  if (!gradient_p<NS>(C, false)) return;
-  C.phase(PH_SETUP);
-  int done = 0;
-  for (int it = 0; it < iters; ++it) {
-    done = it + 1;
-    double Rit[4] = {1.0, 1.0, 1.0, 1.0};
-    bool finite = true;   // Krylov residual norms of this iteration all finite
-    // ---- momentum: assemble, start Krylov, set up M, solve
-    const MatT<T> &AUT = matU<T>(P);
-    const KWorkT<T> &wU = workU<T>(P);
-    C.phase(PH_MOM_ASM);
-    tile_each(C, [&](int i) {
-      double b[NS];
-      momentum_row<NS>(P, i, !piso, b);
-      krylov_init_row<NS, T>(P, P.AU, AUT, wU, b, P.U, i, P.kU.solver);
+  __device__ __forceinline__ bool setup() {
+    const KParams &P = *C.P;
+    const bool mid = (P.grad == GRAD_MIDPOINT);
+    const double nu = P.nu;
+    C.phase(PH_SETUP);
+    grid_each(P.nf, [&](int f) {
+      face_mdot<NS>(P, f);
+      P.pf[f] = face_scalar(P, P.p, f, P.bcP, mid);
+      if (P.model == 1) P.nutf[f] = 0.0;   // initialise_RANS: a fresh face field
+      P.nueff[f] = (P.model == 1) ? nu + 0.0 : nu;
     });
-    if (!C.sync()) return;
-    if (!krylov_start<NS, T>(C, AUT, wU, P.bU, P.kU.solver)) return;
-    int itsU[NS];
-    double rnU[NS];
-    if (!krylov<NS, T>(C, AUT, wU, P.bU, P.kU, P.kU.solver, itsU, rnU)) return;
+    if (!C.sync()) return false;
+    if (!gradient_p<NS>(C, false)) return false;
+    C.phase(PH_SETUP);
+    return true;
+  }
+
+  __device__ __forceinline__ bool before_solve(int k) {
+    const KParams &P = *C.P;
+    const int it = k / ncorr, corr = k - it * ncorr;
+    if (corr == 0) {
+      finite = true;
+      // ---- momentum: assemble, start Krylov, set up M, solve
+      const MatT<T> &AUT = matU<T>(P);
+      const KWorkT<T> &wU = workU<T>(P);
+      C.phase(PH_MOM_ASM);
+      tile_each(C, [&](int i) {
+        double b[NS];
+        momentum_row<NS>(P, i, !piso, b);
+        krylov_init_row<NS, T>(P, P.AU, AUT, wU, b, P.U, i, P.kU.solver);
+      });
+      if (!C.sync()) return false;
+      if (!krylov_start<NS, T>(C, AUT, wU, P.bU, P.kU.solver)) return false;
+      int itsU[NS];
+      double rnU[NS];
+      if (!solve_vector<NS, T>(C, AUT, wU, P.bU, P.kU, itsU, rnU)) return false;
 #pragma unroll
-    for (int d = 0; d < NS; ++d) finite = finite && isfinite(rnU[d]);
-    // run! copy-back: U = x + x0
-    C.phase(PH_UPDATE);
-    tile_each(C, [&](int i) {
+      for (int d = 0; d < NS; ++d) finite = finite && isfinite(rnU[d]);
+      // run! copy-back: U = x + x0
+      C.phase(PH_UPDATE);
+      tile_each(C, [&](int i) {
 #pragma unroll
-      for (int d = 0; d < NS; ++d) {
-        const size_t k = (size_t)i * NS + d;
-        P.U[k] = (double)wU.x[k] + P.U[k];
-      }
-    });
-    if (!C.sync()) return;
-    // ---- residual!(R_ux..), remove_pressure_source!, H!
-    C.phase(PH_RESID);
-    tile_phase<2 * NS>(C, true, [&](int i, double (&v)[2 * NS]) {
-      double y[NS], bb[NS];
-      spmv_row<NS>(P.AU, i, [&](int j, int d) { return P.U[(size_t)j * NS + d]; }, y);
-      const double vol = ldro(P.vol + i);
-      ld<NS>(P.bU, i, bb);
+        for (int d = 0; d < NS; ++d) {
+          const size_t q = (size_t)i * NS + d;
+          P.U[q] = (double)wU.x[q] + P.U[q];
+        }
+      });
+      if (!C.sync()) return false;
+      // ---- residual!(R_ux..), remove_pressure_source!, H!
+      C.phase(PH_RESID);
+      tile_phase<2 * NS>(C, true, [&](int i, double (&v)[2 * NS]) {
+        double y[NS], bb[NS];
+        spmv_row<NS>(P.AU, i, [&](int j, int d) { return P.U[(size_t)j * NS + d]; }, y);
+        const double vol = ldro(P.vol + i);
+        ld<NS>(P.bU, i, bb);
 #pragma unroll
-      for (int d = 0; d < NS; ++d) {
-        const double df = y[d] - bb[d];
-        v[2 * d] = df * df;
-        v[2 * d + 1] = bb[d] * bb[d];
-        bb[d] -= -1.0 * P.gp[(size_t)i * NS + d] * vol;
-      }
-      st<NS>(P.bU, i, bb);
-      H_row<NS>(P, i, bb);
-    });
-    if (!C.sync()) return;
-    {
+        for (int d = 0; d < NS; ++d) {
+          const double df = y[d] - bb[d];
+          v[2 * d] = df * df;
+          v[2 * d + 1] = bb[d] * bb[d];
+          bb[d] -= -1.0 * P.gp[(size_t)i * NS + d] * vol;
+        }
+        st<NS>(P.bU, i, bb);
+        H_row<NS>(P, i, bb);
+      });
+      if (!C.sync()) return false;
       double red[2 * NS];
-      final_sum<2 * NS>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
-#pragma unroll
-      for (int d = 0; d < NS; ++d) Rit[d] = sqrt(red[2 * d] / (double)P.n) / sqrt(red[2 * d + 1]);
+      final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
       if (vbid() == 0 && threadIdx.x == 0) {
 #pragma unroll
         for (int d = 0; d < NS; ++d) {
-          P.R[(size_t)it * 4 + d] = Rit[d];
+          P.R[(size_t)it * 4 + d] = sqrt(red[2 * d] / (double)P.n) / sqrt(red[2 * d + 1]);
           P.kry[(size_t)it * 5 + d] = itsU[d];
         }
+        P.step->finite = finite ? 1 : 0;
       }
-    }
-    const int ncorr = piso ? 2 : 1;
-    for (int corr = 0; corr < ncorr; ++corr) {
-      if (corr > 0) {   // H! again with the corrected U (PISO corrector loop)
-        C.phase(PH_RESID);
-        tile_each(C, [&](int i) {
-          double bb[NS];
-          ld<NS>(P.bU, i, bb);
-          H_row<NS>(P, i, bb);
-        });
-        if (!C.sync()) return;
-      }
-      // interpolate!(rDf, rD); interpolate!(Uf, Hv) + correct_boundaries!
-      C.phase(PH_FACE);
-      grid_each(P.nf, [&](int f) {
-        const double w = ldro(P.wgt + f);
-        const double omw = 1.0 - w;
-        P.rDf[f] = w * P.rD[ldro(P.o1 + f)] + omw * P.rD[ldro(P.o2 + f)];
-        double u[NS];
-        face_vector<NS>(P, P.H, f, u);
-#pragma unroll
-        for (int d = 0; d < NS; ++d) P.UfH[(size_t)f * NS + d] = u[d];
-      });
-      if (!C.sync()) return;
-      // div! + pressure assembly + Krylov start
-      const MatT<T> &APT = matP<T>(P);
-      const KWorkT<T> &wP = workP<T>(P);
-      C.phase(PH_P_ASM);
-      tile_each(C, [&](int i) {
-        double b[1];
-        b[0] = pressure_row<NS>(P, i);
-        krylov_init_row<1, T>(P, P.AP, APT, wP, b, P.p, i, P.kP.solver);
-      });
-      if (!C.sync()) return;
-      if (!krylov_start<1, T>(C, APT, wP, P.bP, P.kP.solver)) return;
-      int itsP[1];
-      double rnP[1];
-      if (!krylov<1, T>(C, APT, wP, P.bP, P.kP, P.kP.solver, itsP, rnP)) return;
-      finite = finite && isfinite(rnP[0]);
-      // run! copy-back then explicit_relaxation!(p, prev, alpha_p)
-      C.phase(PH_UPDATE);
-      tile_each(C, [&](int i) {
-        const double pn = (double)wP.x[i] + P.p[i];
-        const double p0 = P.p[i];
-        P.p[i] = p0 + P.aP * (pn - p0);
-      });
-      if (!C.sync()) return;
-      // residual!(R_p) and the face interpolation of grad!(grad p)
+    } else {   // H! again with the corrected U (PISO corrector loop)
       C.phase(PH_RESID);
-      tile_phase<2>(C, true, [&](int i, double (&v)[2]) {
-        double y[1];
-        spmv_row<1>(P.AP, i, [&](int j, int d) { return P.p[j]; }, y);
-        const double bb = P.bP[i];
-        const double df = y[0] - bb;
-        v[0] = df * df;
-        v[1] = bb * bb;
+      tile_each(C, [&](int i) {
+        double bb[NS];
+        ld<NS>(P.bU, i, bb);
+        H_row<NS>(P, i, bb);
       });
-      grid_each(P.nf, [&](int f) { P.pf[f] = face_scalar(P, P.p, f, P.bcP, mid); });
-      if (!C.sync()) return;
-      {
-        double red[2];
-        final_sum<2>(C.part_r(), P.ntiles, C.sm, C.sm_out, red);
-        Rit[3] = sqrt(red[0] / (double)P.n) / sqrt(red[1]);
-        if (vbid() == 0 && threadIdx.x == 0) {
-          P.R[(size_t)it * 4 + 3] = Rit[3];
-          P.kry[(size_t)it * 5 + 3] = itsP[0];
-        }
-      }
-      if (!gradient_p<NS>(C, true)) return;
-      // interpolate!(Uf, U) + correct_boundaries! + flux!(mdotf, Uf)
-      C.phase(PH_FACE);
-      grid_each(P.nf, [&](int f) { face_mdot<NS>(P, f); });
-      if (!C.sync()) return;
-      if (P.model == 1 && !turbulence<NS, T>(C)) return;
+      if (!C.sync()) return false;
     }
+    // interpolate!(rDf, rD); interpolate!(Uf, Hv) + correct_boundaries!
+    C.phase(PH_FACE);
+    grid_each(P.nf, [&](int f) {
+      const double w = ldro(P.wgt + f);
+      const double omw = 1.0 - w;
+      P.rDf[f] = w * P.rD[ldro(P.o1 + f)] + omw * P.rD[ldro(P.o2 + f)];
+      double u[NS];
+      face_vector<NS>(P, P.H, f, u);
+#pragma unroll
+      for (int d = 0; d < NS; ++d) P.UfH[(size_t)f * NS + d] = u[d];
+    });
+    if (!C.sync()) return false;
+    // div! + pressure assembly + Krylov start
+    const MatT<T> &APT = matP<T>(P);
+    const KWorkT<T> &wP = workP<T>(P);
+    C.phase(PH_P_ASM);
+    tile_each(C, [&](int i) {
+      double b[1];
+      b[0] = pressure_row<NS>(P, i);
+      krylov_init_row<1, T>(P, P.AP, APT, wP, b, P.p, i, P.kP.solver);
+    });
+    if (!C.sync()) return false;
+    return krylov_start<1, T>(C, APT, wP, P.bP, P.kP.solver);
+  }
+
+  // After solve k with `its` iterations and residual norm rn; stop: the run
+  // ends with this iteration.
+  __device__ __forceinline__ bool after_solve(int k, int its, double rn, bool &stop) {
+    const KParams &P = *C.P;
+    const bool mid = (P.grad == GRAD_MIDPOINT);
+    const int it = k / ncorr, corr = k - it * ncorr;
+    const KWorkT<T> &wP = workP<T>(P);
+    finite = finite && isfinite(rn);
+    // run! copy-back then explicit_relaxation!(p, prev, alpha_p)
+    C.phase(PH_UPDATE);
+    tile_each(C, [&](int i) {
+      const double pn = (double)wP.x[i] + P.p[i];
+      const double p0 = P.p[i];
+      P.p[i] = p0 + P.aP * (pn - p0);
+    });
+    if (!C.sync()) return false;
+    // residual!(R_p) and the face interpolation of grad!(grad p)
+    C.phase(PH_RESID);
+    tile_phase<2>(C, true, [&](int i, double (&v)[2]) {
+      double y[1];
+      spmv_row<1>(P.AP, i, [&](int j, int d) { return P.p[j]; }, y);
+      const double bb = P.bP[i];
+      const double df = y[0] - bb;
+      v[0] = df * df;
+      v[1] = bb * bb;
+    });
+    grid_each(P.nf, [&](int f) { P.pf[f] = face_scalar(P, P.p, f, P.bcP, mid); });
+    if (!C.sync()) return false;
+    double red[2];
+    final_sum<2>(C.part_r(), P.ntiles, s_sm, s_out, red);
+    const double Rp = sqrt(red[0] / (double)P.n) / sqrt(red[1]);
+    if (vbid() == 0 && threadIdx.x == 0) {
+      P.R[(size_t)it * 4 + 3] = Rp;
+      P.kry[(size_t)it * 5 + 3] = its;
+      P.step->finite = finite ? 1 : 0;
+    }
+    if (!gradient_p<NS>(C, true)) return false;
+    // interpolate!(Uf, U) + correct_boundaries! + flux!(mdotf, Uf)
+    C.phase(PH_FACE);
+    grid_each(P.nf, [&](int f) { face_mdot<NS>(P, f); });
+    if (!C.sync()) return false;
+    if constexpr (NS == 2) {   // k-omega is a 2D model (xcal_case_setup refuses it in 3D)
+      if (P.model == 1 && !turbulence<NS, T>(C)) return false;
+    }
+    if (corr + 1 < ncorr) return true;
+    const bool lead = vbid() == 0 && threadIdx.x == 0;
     // XCAL_FLAG_ABORT_ON_NAN (no reference counterpart): stop a diverged run.
     // The residuals R_* themselves may be 0/0 = NaN on a healthy run (a zero
     // right-hand side, e.g. uy at the first iteration), so the test uses the
     // Krylov residual norms, which are finite whenever A, b and x0 are.
-    if (P.abort_nan) {
-      if (!finite) {
-        if (vbid() == 0 && threadIdx.x == 0) P.bar->nonfinite = 1;
-        break;
+    if (P.abort_nan && !finite) {
+      if (lead) P.bar->nonfinite = 1;
+      stop = true;
+    } else if (!piso) {
+      // convergence test (Solvers_1_SIMPLE.jl:200-215); every CTA reads the
+      // same residuals (CTA 0 stored the momentum ones several barriers ago),
+      // so all take the same branch
+      bool c = Rp <= P.conv;
+#pragma unroll
+      for (int d = 0; d < NS; ++d) c = c && (P.R[(size_t)it * 4 + d] <= P.conv);
+      stop = c;
+    }
+    if (lead) *P.done = it + 1;
+    return true;
+  }
+};
+
+// The chain of a run.  step < 0: all of it.  Otherwise one link, for large
+// meshes, whose pressure solve is a kernel of its own (xcal_cg_kernel): launch
+// `step` does what follows solve step-1 and what leads to solve `step`, and
+// P.step carries the solve's results and the state of the run between them.
+template <int NS, typename T>
+__device__ __forceinline__ void simple_program(Ctx &C, int iters, bool piso, int step) {
+  const KParams &P = *C.P;
+  Simple<NS, T> S{C, piso, piso ? 2 : 1, true};
+  const int total = iters * S.ncorr;
+  int its[1] = {0};
+  double rn[1] = {0.0};
+  if (step > 0) {
+    S.finite = P.step->finite != 0;
+    its[0] = P.step->its;
+    rn[0] = P.step->rnorm;
+  } else if (!S.setup()) {
+    return;
+  }
+  for (int k = max(step, 0);; ++k) {
+    if (k > 0) {
+      bool stop = false;
+      if (!S.after_solve(k - 1, its[0], rn[0], stop)) return;
+      if (stop) {
+        if (vbid() == 0 && threadIdx.x == 0) P.step->stop = 1;
+        return;
       }
     }
-    if (!piso) {
-      // convergence test (Solvers_1_SIMPLE.jl:200-215); every CTA holds the
-      // same residual values, so all take the same branch
-      const double conv = P.conv;
-      bool c = true;
-#pragma unroll
-      for (int d = 0; d < NS; ++d) c = c && (Rit[d] <= conv);
-      c = c && (Rit[3] <= conv);
-      if (c) break;
+    if (k == total) return;
+    if (!S.before_solve(k)) return;
+    if (step >= 0) {
+      if (vbid() == 0 && threadIdx.x == 0) P.step->pw = C.pw;
+      return;
     }
+    if (!solve_scalar<NS, T>(C, matP<T>(P), workP<T>(P), P.bP, P.kP, its, rn)) return;
   }
-  if (vbid() == 0 && threadIdx.x == 0) *P.done = done;
 }
 
 __device__ __forceinline__ void solve_program(Ctx &C) {
@@ -1866,7 +2301,7 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
   cfg.rtol = P.solve_rtol;
   int its[1];
   double rn[1];
-  if (!krylov<1, double>(C, P.AU, P.wU, P.sb, cfg, P.solve_solver, its, rn)) return;
+  if (!solve_scalar<1, double>(C, P.AU, P.wU, P.sb, cfg, its, rn)) return;
   tile_each(C, [&](int i) { P.U[i] = P.wU.x[i] + P.U[i]; });
   if (vbid() == 0 && threadIdx.x == 0) {
     P.solve_out[0] = (double)its[0];
@@ -1877,22 +2312,10 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
 
 }  // namespace
 
-// KParams is passed by value: the fields live in the kernel's constant
-// parameter bank instead of occupying registers.  T is the scalar type of
-// the Krylov iterations (double: FP64 path; float: mixed path).  MB is the
-// number of resident CTAs per SM the register budget is sized for: 2 (128
-// registers, few spills) suits meshes with about one tile per CTA, where a
-// phase is barrier-latency bound; 4 (64 registers, more spills, twice the
-// warps in flight) suits large meshes, where a phase is memory-latency bound.
-template <int NS, typename T, int MB>
-__global__ void __launch_bounds__(TPB, MB) xcal_program_kernel(const __grid_constant__ KParams prm, int prog, int iters) {
-  __shared__ double sm[8 * MAXK];
-  __shared__ double sm_out[MAXK];
-  __shared__ double ws[MAXTL * MAXK * 8];
-  __shared__ int sm_ok;
-  __shared__ unsigned long long pacc[2 * NPH];
-  Ctx C;
-  C.P = &prm;
+// State of a launch whose CTAs are all of one group.
+__device__ __forceinline__ void launch_begin(Ctx &C, const KParams &prm) {
+  ctx_mesh(C, prm);
+  copies_init(false);
   C.S.bar = prm.bar;
   C.S.mode = prm.mode;
   C.S.nb = gridDim.x;
@@ -1904,27 +2327,347 @@ __global__ void __launch_bounds__(TPB, MB) xcal_program_kernel(const __grid_cons
   C.S.extra = (unsigned)prm.bar_extra;
   C.S.timeout_ns = prm.bar_timeout_ns ? prm.bar_timeout_ns : BARRIER_TIMEOUT_NS;
   C.S.epoch = 0;
-  C.S.ok = &sm_ok;
   C.part = prm.part;
   C.pw = 0;
   C.rev = 0;
-  C.sm = sm;
-  C.sm_out = sm_out;
-  C.ws = ws;
   C.timers = prm.phase != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
   C.tag = PH_SETUP;
-  C.pacc = pacc;
   if (C.timers) {
-    for (int k = 0; k < 2 * NPH; ++k) pacc[k] = 0ull;
+    for (int k = 0; k < 2 * NPH; ++k) s_pacc[k] = 0ull;
     C.t_last = clock64();
   }
+}
+// The timers are added up over the launches of a run.  `again`: another launch
+// with the same barrier word follows, so the last CTA out clears its count.
+__device__ __forceinline__ void launch_end(Ctx &C, const KParams &prm, bool again) {
+  if (C.timers)
+    for (int k = 0; k < 2 * NPH; ++k) prm.phase[k] += s_pacc[k];
+  if (!again) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned out = atomicAdd(&prm.bar->exits, 1u);
+    if (out + 1u == gridDim.x) {
+      prm.bar->count = 0ull;
+      prm.bar->exits = 0u;
+    }
+  }
+}
+
+#if defined(XCAL_CG)
+// The pressure solve of a large mesh (rows of which the CTAs cannot keep in
+// shared memory) as a kernel of its own.  Its phases stream the matrix with a
+// few dependent gathers per row, and what hides their latency is warps: this
+// kernel needs few registers, so MB = 8 CTAs fit an SM where the program's
+// register budget allows 4.
+template <typename T, int WT, int MB>
+__global__ void __launch_bounds__(TPB, MB) xcal_cg_kernel(const __grid_constant__ KParams prm) {
+  if (ld_volatile_i32(&prm.bar->err) || ld_volatile_i32(&prm.step->stop)) return;
+  Ctx C;
+  launch_begin(C, prm);
+  C.pw = prm.step->pw;
+  int its;
+  double rn;
+  if (cg_two_level<T, WT, false>(C, matP<T>(prm), workP<T>(prm), prm.kP, its, rn) && vbid() == 0 && threadIdx.x == 0) {
+    prm.step->its = its;
+    prm.step->rnorm = rn;
+  }
+  launch_end(C, prm, true);
+}
+
+// The pressure solve of a small mesh as one cluster of CTAs holding all of it
+// in shared memory: matrix rows, preconditioner and Krylov vectors.  A row's
+// neighbours are read through distributed shared memory (their addresses are
+// worked out once, in place of the column indices), tile sums are stored
+// straight into every CTA's copy of the partials, and the barrier is the
+// cluster's own, so no phase goes through L2.  Row arithmetic and sums are
+// those of cg_two_level.
+//
+// A CTA holds a chunk of the tiles with level-0 rows and the same chunk of
+// the others: its rows are close together in the mesh, so most neighbours
+// are its own, and all CTAs work in each phase.  Four tiles at a time, one
+// per 256 threads.
+enum { CV_Z = 0, CV_P = 1, CV_R = 3, CV_Q = 5, CV_D = 6, CV_X = 7 };   // vectors (p and r twice)
+static_assert(CV_X + 1 == CGC_VECTORS, "vectors of a row");
+
+__device__ __forceinline__ unsigned cluster_addr(unsigned a, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ double ld_cluster(unsigned a, double) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float ld_cluster(unsigned a, float) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void st_cluster(unsigned a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, int WT>
+__global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __grid_constant__ KParams prm, int slots) {
+  __shared__ double part[2][CGC_TILES];
+  __shared__ double ws[CGC_SLOTS * 8];
+  __shared__ double sm[8];
+  if (ld_volatile_i32(&prm.bar->err) || ld_volatile_i32(&prm.step->stop)) return;
+  constexpr double EPS = 2.220446049250313e-16;
+  const MatT<T> &A = matP<T>(prm);
+  const KWorkT<T> &w = workP<T>(prm);
+  const int n = prm.n, n0 = prm.n0, np = prm.np, nt = prm.ntiles;
+  const int W = WT < WUNROLL ? WT : A.W;
+  const int tid = threadIdx.x, lane = tid & 31, tl = tid >> 8, r = tid & 255, wt = (tid >> 5) & 7;
+  const int G = gridDim.x, b = blockIdx.x;
+  // tiles [0, N0) hold level-0 rows, the rest only level-1 rows; tile N0-1 may hold both
+  const int N0 = (n0 - 1) / TILE + 1, N1 = nt - N0;
+  const int a0 = chunk(b, N0, G), k0 = chunk(b + 1, N0, G) - a0;                // own level-0 tiles: slots [0, k0)
+  const int a1 = N0 + chunk(b, N1, G), cnt = k0 + chunk(b + 1, N1, G) - chunk(b, N1, G);   // the others: [k0, cnt)
+  const int L = slots * TILE;
+  T *vec = (T *)s_dyn, *val = vec + (size_t)CGC_VECTORS * L;
+  unsigned *adr = (unsigned *)(val + (size_t)W * L);
+  const unsigned vec0 = smem_u32(vec);
+  auto tile_of = [&](int s) { return s < k0 ? a0 + s : a1 + (s - k0); };
+  const bool timer = prm.phase != nullptr && b == 0 && tid == 0;
+  long long t_last = timer ? clock64() : 0, acc[2] = {0, 0}, num[2] = {0, 0};
+  auto tick = [&](int what) {
+    if (timer) {
+      const long long t = clock64();
+      acc[what] += t - t_last;
+      num[what] += 1;
+      t_last = t;
+    }
+  };
+  // rows into shared memory; entry k's neighbour as the address of its z in
+  // the cluster, with bit 0 for the diagonal and bit 1 for padding
+  for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+    const int l = s * TILE + r, i = tile_of(s) * TILE + r;
+    const bool on = i < n;
+    vec[CV_Z * L + l] = on ? w.v[0][i] : T(0);
+    vec[CV_R * L + l] = on ? w.r[0][i] : T(0);
+    vec[CV_D * L + l] = on ? A.Dinv[i] : T(0);
+    vec[CV_X * L + l] = T(0);
+    const unsigned own = vec0 + (unsigned)(l * sizeof(T));
+    for (int k = 0; k < W; ++k) {
+      const int c = A.col[(size_t)k * np + i];
+      val[(size_t)k * L + l] = A.val[(size_t)k * np + i];
+      unsigned a = cluster_addr(own, b) | 2u;
+      if (c >= 0) {
+        const int t = c / TILE, g = t < N0 ? t : t - N0, N = t < N0 ? N0 : N1;
+        const int o = (int)(((long long)(g + 1) * G - 1) / N);   // its CTA
+        const int slot = g - chunk(o, N, G) + (t < N0 ? 0 : chunk(o + 1, N0, G) - chunk(o, N0, G));
+        a = cluster_addr(vec0 + (unsigned)((slot * TILE + c % TILE) * sizeof(T)), o) | (c == i ? 1u : 0u);
+      }
+      adr[(size_t)k * L + l] = a;
+    }
+  }
+  int par = 0;
+  {
+    const double *p0 = prm.part + (size_t)(prm.step->pw ^ 1) * MAXK * nt;
+    if (tid < nt) part[par][tid] = p0[tid];
+  }
+  cluster_sync();
+  // canonical sum of the tiles' partials (final_sum's tree; one tile per lane)
+  auto total = [&]() -> double {
+    if (tid < TPB) {
+      double a = tid < nt ? part[par][tid] : 0.0;
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) a = a + __shfl_down_sync(0xffffffffu, a, off);
+      if (lane == 0) sm[tid >> 5] = a;
+    }
+    __syncthreads();
+    par ^= 1;
+    double x0 = sm[0] + sm[4], x1 = sm[1] + sm[5];
+    const double x2 = sm[2] + sm[6], x3 = sm[3] + sm[7];
+    x0 = x0 + x2;
+    x1 = x1 + x3;
+    return x0 + x1;
+  };
+  auto stage = [&](int s, double v) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) ws[s * 8 + wt] = v;
+  };
+  // every own tile's sum to every CTA, then the barrier
+  auto exchange = [&]() {
+    __syncthreads();
+    for (int q = tid; q < cnt * G; q += CGC_TPB) {
+      const int s = q / G;
+      const double *ww = ws + s * 8;
+      double x0 = ww[0] + ww[4], x1 = ww[1] + ww[5];
+      const double x2 = ww[2] + ww[6], x3 = ww[3] + ww[7];
+      x0 = x0 + x2;
+      x1 = x1 + x3;
+      st_cluster(cluster_addr(smem_u32(&part[par][tile_of(s)]), q - s * G), x0 + x1);
+    }
+    cluster_sync();
+  };
+
+  double s0 = total();
+  const double sgn = (s0 < 0.0) ? -1.0 : 1.0;
+  double gamma = sgn * s0, rnorm = sqrt(gamma), alpha = 0.0, beta = 0.0, pn2 = gamma, eps = 0.0;
+  int its = 0;
+  bool active = false;
+  const KCfg &cfg = prm.kP;
+  if (gamma != 0.0) {
+    eps = cfg.atol + cfg.rtol * rnorm;
+    active = !(rnorm <= eps || 0 >= cfg.itmax);
+  }
+  int ro = CV_R, rn = CV_R + 1, po = CV_Z, pn = CV_P, pspare = CV_P + 1;   // first direction: as in cg_two_level
+  bool pending = false;
+  const int sB = (k0 > 0 && tile_of(k0 - 1) == N0 - 1 && n0 < N0 * TILE) ? k0 - 1 : k0;   // first slot with level-1 rows
+  while (active) {
+    // A
+    {
+      const unsigned opo = (unsigned)(po * L * sizeof(T));
+      for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+        const int l = s * TILE + r;
+        T y = T(0), pi = T(0), poi = T(0);
+#pragma unroll
+        for (int k = 0; k < WT; ++k) {
+          const int kk = (WT < WUNROLL || k < W) ? k : W - 1;
+          const unsigned a = (WT < WUNROLL || k < W) ? adr[kk * L + l] : 2u | (unsigned)vec0;
+          const unsigned ad = (a & 2u) ? adr[l] & ~3u : a & ~3u;
+          const T oj = ld_cluster(ad + opo, T()), pj = vaxpy<T>(ld_cluster(ad, T()), beta, oj);
+          const T t = y + val[kk * L + l] * pj;
+          y = (a & 2u) ? y : t;
+          if (a & 1u) {
+            pi = pj;
+            poi = oj;
+          }
+        }
+        vec[CV_X * L + l] = vaxpy<T>(vec[CV_X * L + l], alpha, poi);
+        vec[pn * L + l] = pi;
+        vec[CV_Q * L + l] = y;
+        stage(s, (double)pi * (double)y);
+      }
+      pending = false;
+      exchange();
+      s0 = total();
+      tick(0);
+    }
+    const double pAp = sgn * s0;
+    if (pAp <= EPS * pn2 && fabs(pAp) <= EPS * pn2) break;   // zero curvature: stop
+    alpha = gamma / pAp;
+    const unsigned oro = (unsigned)(ro * L * sizeof(T)), oq = (unsigned)(CV_Q * L * sizeof(T)),
+                   od = (unsigned)(CV_D * L * sizeof(T));
+    // B
+    for (int s = sB + tl; s < cnt; s += CGC_TPB / TILE) {
+      const int l = s * TILE + r, i = tile_of(s) * TILE + r;
+      double rz = 0.0;
+      if (i < n && i >= n0) {
+        const T ri = vaxpy<T>(vec[ro * L + l], -alpha, vec[CV_Q * L + l]);
+        T o = ri;
+#pragma unroll
+        for (int k = 0; k < WT - 1; ++k) {
+          const int kk = (WT < WUNROLL || k < W - 1) ? k : 0;
+          const unsigned a = (WT < WUNROLL || k < W - 1) ? adr[kk * L + l] : 2u;
+          const bool use = (a & 3u) == 0u;
+          const unsigned ad = use ? a : adr[l] & ~3u;
+          const T t = o - val[kk * L + l] * vaxpy<T>(ld_cluster(ad + oro, T()), -alpha, ld_cluster(ad + oq, T())) *
+                              ld_cluster(ad + od, T());
+          o = use ? t : o;
+        }
+        o = o * vec[CV_D * L + l];
+        vec[rn * L + l] = ri;
+        vec[CV_Z * L + l] = o;
+        rz = (double)ri * (double)o;
+      }
+      if (s >= k0) stage(s, rz);
+    }
+    cluster_sync();
+    tick(1);
+    // C
+    for (int s = tl; s < k0; s += CGC_TPB / TILE) {
+      const int l = s * TILE + r, i = tile_of(s) * TILE + r;
+      double rz = 0.0;
+      if (i < n0) {
+        const T ri = vaxpy<T>(vec[ro * L + l], -alpha, vec[CV_Q * L + l]);
+        const T di = vec[CV_D * L + l];
+        T o = ri * di;
+#pragma unroll
+        for (int k = 1; k < WT; ++k) {
+          const int kk = (WT < WUNROLL || k < W) ? k : W - 1;
+          const unsigned a = (WT < WUNROLL || k < W) ? adr[kk * L + l] : 2u;
+          const bool use = (a & 3u) == 0u;
+          const unsigned ad = use ? a : adr[l] & ~3u;
+          const T t = o - val[kk * L + l] * ld_cluster(ad, T()) * di;
+          o = use ? t : o;
+        }
+        vec[rn * L + l] = ri;
+        vec[CV_Z * L + l] = o;
+        rz = (double)ri * (double)o;
+      } else if (i < n) {   // level-1 rows of the tile that holds both levels
+        rz = (double)vec[rn * L + l] * (double)vec[CV_Z * L + l];
+      }
+      stage(s, rz);
+    }
+    exchange();
+    s0 = total();
+    tick(1);
+    const double gn = sgn * s0;
+    rnorm = sqrt(gn);
+    const bool solved = (rnorm <= eps) || (rnorm + 1.0 <= 1.0);
+    if (!solved) {
+      beta = gn / gamma;
+      pn2 = gn + (beta * beta) * pn2;
+      gamma = gn;
+    }
+    its += 1;
+    active = !(solved || its >= cfg.itmax);
+    pending = true;
+    int tp = ro;
+    ro = rn;
+    rn = tp;
+    tp = pn;
+    pn = pspare;
+    pspare = tp;
+    po = tp;
+  }
+  for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+    const int l = s * TILE + r, i = tile_of(s) * TILE + r;
+    const T x = vec[CV_X * L + l];
+    if (i < n) w.x[i] = pending ? vaxpy<T>(x, alpha, vec[po * L + l]) : x;
+  }
+  if (b == 0 && tid == 0) {
+    prm.step->its = its;
+    prm.step->rnorm = rnorm;
+  }
+  if (timer) {
+    prm.phase[PH_KRY_SPMV] += acc[0];
+    prm.phase[PH_KRY_PREC] += acc[1];
+    prm.phase[NPH + PH_KRY_SPMV] += num[0];
+    prm.phase[NPH + PH_KRY_PREC] += num[1];
+  }
+  cluster_sync();   // no CTA leaves while another may still reach its memory
+}
+#endif
+
+// KParams is passed by value: the fields live in the kernel's constant
+// parameter bank instead of occupying registers.  T is the scalar type of
+// the Krylov iterations (double: FP64 path; float: mixed path).  MB is the
+// number of resident CTAs per SM the register budget is sized for: 2 (128
+// registers, few spills) suits meshes with about one tile per CTA, where a
+// phase is barrier-latency bound; 4 (64 registers, more spills, twice the
+// warps in flight) suits large meshes, where a phase is memory-latency bound.
+template <int NS, typename T, int MB>
+__global__ void __launch_bounds__(TPB, MB) xcal_program_kernel(const __grid_constant__ KParams prm, int prog, int iters,
+                                                               int step) {
+  if (step > 0 && (ld_volatile_i32(&prm.bar->err) || ld_volatile_i32(&prm.step->stop))) return;
+  Ctx C;
+  launch_begin(C, prm);
   if (prog == PROG_SOLVE) {
     if constexpr (NS == 1 && sizeof(T) == 8) solve_program(C);
   } else {
-    if constexpr (NS >= 2) simple_program<NS, T>(C, iters, prog == PROG_PISO);
+    if constexpr (NS >= 2) simple_program<NS, T>(C, iters, prog == PROG_PISO, step);
   }
-  if (C.timers)
-    for (int k = 0; k < 2 * NPH; ++k) prm.phase[k] = pacc[k];
+  launch_end(C, prm, step >= 0);
 }
 
 // ------------------------------------------------------------- serving
@@ -1953,16 +2696,12 @@ __device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned *p, unsigned v)
 
 template <int NS, typename T, int MB>
 __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, const ServeCtl *ctl) {
-  __shared__ double sm[8 * MAXK];
-  __shared__ double sm_out[MAXK];
-  __shared__ double ws[MAXTL * MAXK * 8];
-  __shared__ int sm_ok;
-  __shared__ unsigned long long pacc[2 * NPH];
   __shared__ ServeJob sJ;   // the job record, read once per job
   __shared__ const ServeJob *s_job;
   __shared__ int s_cmd;
   static_assert(sizeof(ServeJob) % 8 == 0, "job record copied in 8-byte words");
   ServeMail *m = mail + blockIdx.x;
+  unsigned jobs = 0;
   unsigned long long seen = 0;
   if (threadIdx.x == 0) seen = *(volatile unsigned long long *)&m->ack;
   for (;;) {
@@ -2028,25 +2767,21 @@ __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, co
         dst[c16 + q] = zero;
     }
     Ctx C;
-    C.P = &sP;
+    ctx_mesh(C, sP);
+    copies_init(jobs++ > 0);
     C.S.bar = sP.bar;
     C.S.mode = SYNC_GRID;
     C.S.nb = G;
     C.S.extra = 0;
     C.S.timeout_ns = BARRIER_TIMEOUT_NS;
     C.S.epoch = 0;
-    C.S.ok = &sm_ok;
     C.part = sP.part;
     C.pw = 0;
     C.rev = 0;
-    C.sm = sm;
-    C.sm_out = sm_out;
-    C.ws = ws;
     C.timers = false;
     C.tag = PH_SETUP;
-    C.pacc = pacc;
     C.t_last = 0;
-    if (C.sync()) simple_program<NS, T>(C, J.iters, J.prog == PROG_PISO);
+    if (C.sync()) simple_program<NS, T>(C, J.iters, J.prog == PROG_PISO, -1);
     C.sync();   // the run's results (fields, histories, done) complete
     // results to pinned host memory, this CTA's share
     {
@@ -2088,13 +2823,24 @@ __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, co
 #ifndef XCAL_MB
 #define XCAL_MB 2
 #endif
-#if defined(XCAL_SERVE_ONLY)
+#if defined(XCAL_CG)
+const void *XCAL_CAT(cg_kernel_, XCAL_INST)(int W) {
+  if (W == 5) return (const void *)xcal_cg_kernel<XCAL_T, 5, XCAL_MB>;
+  if (W == 7) return (const void *)xcal_cg_kernel<XCAL_T, 7, XCAL_MB>;
+  return (const void *)xcal_cg_kernel<XCAL_T, WUNROLL, XCAL_MB>;
+}
+const void *XCAL_CAT(cgc_kernel_, XCAL_INST)(int W) {
+  if (W == 5) return (const void *)xcal_cg_cluster_kernel<XCAL_T, 5>;
+  if (W == 7) return (const void *)xcal_cg_cluster_kernel<XCAL_T, 7>;
+  return (const void *)xcal_cg_cluster_kernel<XCAL_T, WUNROLL>;
+}
+#elif defined(XCAL_SERVE_ONLY)
 template __global__ void xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB>(ServeMail *, const ServeCtl *);
 const void *XCAL_CAT(serve_kernel_, XCAL_INST)() {
   return (const void *)xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB>;
 }
 #else
-template __global__ void xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB>(const __grid_constant__ KParams, int, int);
+template __global__ void xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB>(const __grid_constant__ KParams, int, int, int);
 const void *XCAL_CAT(program_kernel_, XCAL_INST)() {
   return (const void *)xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB>;
 }

@@ -8,7 +8,21 @@ namespace xcal {
 // occ selects the build: 0 = two resident CTAs per SM (128 registers),
 // 1 = four (64 registers); the NS = 1 standalone-solve program has only the first.
 cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, const KParams *hparams, int prog,
-                           int iters, cudaStream_t stream);
+                           int iters, int step, cudaStream_t stream);
+// The pressure solve between two steps of a run (two-level numbering, row
+// width at most WUNROLL), on cg_blocks CTAs.
+cudaError_t launch_cg(int mixed, int nblocks, const KParams *hparams, cudaStream_t stream);
+int cg_blocks(int mixed, int W, int device);
+// The same solve in one cluster that holds the mesh in shared memory: its CTAs
+// and the tiles of the largest share; 0 CTAs when the mesh does not fit.
+struct CgCluster {
+  int ctas, slots;
+};
+CgCluster cg_cluster(int mixed, int W, int n0, int ntiles);
+cudaError_t launch_cg_cluster(int mixed, const CgCluster &form, const KParams *hparams, cudaStream_t stream);
+// Matrix tiles of the launch's dynamic shared memory ring (KParams::ring).
+int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks);
+size_t serve_dynamic_smem();
 int max_coresident_blocks(int ns, int occ, int device);
 int max_cluster_blocks(int ns, int occ = 0);
 const void *program_kernel_ptr(int ns, int mixed, int occ);

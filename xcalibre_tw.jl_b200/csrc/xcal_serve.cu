@@ -441,7 +441,7 @@ void sched_main(xcal_server s) {
 
 int launch_server_kernel(xcal_server s) {
   void *args[2] = {(void *)&s->mail_dev, (void *)&s->ctl_dev};
-  cudaError_t e = cudaLaunchCooperativeKernel(s->kfn, dim3(s->grid), dim3(xcal::TPB), args, 0, s->kstream);
+  cudaError_t e = cudaLaunchCooperativeKernel(s->kfn, dim3(s->grid), dim3(xcal::TPB), args, xcal::serve_dynamic_smem(), s->kstream);
   if (e != cudaSuccess) return XCAL_ERR_CUDA;
   if (cudaEventRecord(s->kdone, s->kstream) != cudaSuccess) return XCAL_ERR_CUDA;
   s->kernel_live = true;
