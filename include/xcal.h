@@ -216,17 +216,16 @@ int xcal_piso_run(xcal_ctx ctx, int32_t iterations, double *R_ux, double *R_uy,
 /* Autotuner (no reference counterpart): times `iterations` SIMPLE iterations
  * of the context's case in each launch form that computes the same values
  * (program build for 2 or 4 CTAs per SM, CTA count, hardware cluster or grid
- * barrier, CG with M^-1 inside its x/r phase), keeps the fastest for the
- * context, and remembers it for later contexts whose mesh falls in the same
+ * barrier), keeps the fastest for the context, and remembers it for later contexts whose mesh falls in the same
  * class (components, power-of-two bucket of 256-cell tiles, matrix row width,
  * precision).  The case's fields are restored afterwards, so the tuning runs
  * leave no trace in the results.  Environment overrides (XCAL_SYNC, XCAL_OCC,
- * XCAL_NBLOCKS, XCAL_CG_FUSE) take precedence over a remembered choice. */
+ * XCAL_NBLOCKS) take precedence over a remembered choice. */
 typedef struct {
   int32_t mode;             /* 1 hardware cluster barrier, 2 grid barrier */
   int32_t ctas;             /* CTAs of the launch */
   int32_t ctas_per_sm;      /* build of the program: 2 or 4 resident CTAs per SM */
-  int32_t cg_fused;         /* 1: CG applies M^-1 inside its x/r phase */
+  int32_t cg_fused;         /* always 0 (CG with M^-1 inside its x/r phase was never the faster form) */
   int32_t candidates;       /* forms timed */
   int32_t pad;
   double ms_per_iteration;  /* the chosen form */

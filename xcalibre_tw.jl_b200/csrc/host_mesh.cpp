@@ -550,6 +550,28 @@ void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reord
 }
 
 // ---------------------------------------------------------- device layout
+LevelLists level_lists(const std::vector<int> &flev, const std::vector<int> &blev, int n, int nfl, int nbl) {
+  LevelLists L;
+  if ((nfl <= 2 && nbl <= 2) || n > (long long)SWEEP_WIDTH * std::min(nfl, nbl)) return L;
+  auto list = [&](const std::vector<int> &lev, int nl, std::vector<int> &row) {
+    std::vector<int> ptr(nl + 1, 0);
+    for (int i = 0; i < n; ++i) ptr[lev[i] + 1]++;
+    for (int l = 0; l < nl; ++l) ptr[l + 1] += ptr[l];
+    int count = 0;
+    for (int l = 0; l < nl; ++l) {
+      L.ptr.push_back(count);
+      for (int p = ptr[l]; p < ptr[l + 1]; p += 32, ++count)
+        L.items.insert(L.items.end(), {p, std::min(p + 32, ptr[l + 1])});
+    }
+    L.ptr.push_back(count);
+    row.resize(n);
+    for (int i = 0; i < n; ++i) row[ptr[lev[i]]++] = i;
+  };
+  list(flev, nfl, L.frow);
+  list(blev, nbl, L.brow);
+  return L;
+}
+
 int two_level_rows(const std::vector<int> &flev, int n, int nfl, int nbl) {
   if (nfl != 2 || nbl != 2) return 0;
   int n0 = 0;
@@ -657,6 +679,7 @@ int prepare(const HostMesh &M, Prep &P, std::string &err) {
   P.nfl = P.nbl = 1;
   for (int i = 0; i < n; ++i) { P.nfl = std::max(P.nfl, P.flev[i] + 1); P.nbl = std::max(P.nbl, P.blev[i] + 1); }
   P.n0 = two_level_rows(P.flev, n, P.nfl, P.nbl);
+  P.lists = level_lists(P.flev, P.blev, n, P.nfl, P.nbl);
   P.flev.resize(P.np, 0);
   P.blev.resize(P.np, 0);
   P.o1.resize(nf); P.o2.resize(nf);

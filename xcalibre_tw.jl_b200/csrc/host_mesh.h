@@ -36,6 +36,19 @@ void renumber_perm(const HostMesh &M, int mode, std::vector<int64_t> &perm);
 void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reorder_faces,
                 HostMesh &out);
 
+// Lists of the sweeps by one CTA (KParams::frow, brow, items, lptr): rows by
+// forward and by backward level, items of up to 32 rows of a level, the first
+// item of each level.  Empty where the grid sweeps level by level: two levels,
+// or levels of more than SWEEP_WIDTH rows on average.
+// (ms per SIMPLE iteration, grid / one CTA, by average rows per level: BFS 5k
+// 17: 188 / 117; cavity 40^2 20: 19 / 12; cavity 80^2 40: 84 / 70; hex 12^3 51:
+// 6.0 / 4.5; cavity 160^2 80: 172 / 211; hex 20^3 138: 9.7 / 14.6.)
+constexpr int SWEEP_WIDTH = 56;
+struct LevelLists {
+  std::vector<int> frow, brow, items, ptr;
+};
+LevelLists level_lists(const std::vector<int> &flev, const std::vector<int> &blev, int n, int nfl, int nbl);
+
 // Device-ready integer structures built from a (renumbered) mesh.  Matrix and
 // per-cell face lists use an ELL layout padded to np = 256*ceil(n/256) rows:
 // entry k of row i sits at k*np + i (coalesced across a warp); unused entries
@@ -51,6 +64,7 @@ struct Prep {
   std::vector<int> flev, blev;
   int nfl = 0, nbl = 0;
   int n0 = 0;                                // two_level_rows
+  LevelLists lists;
   std::vector<int> o1, o2;
 };
 int prepare(const HostMesh &M, Prep &P, std::string &err);

@@ -197,17 +197,6 @@ struct DevSink : Sink {
 };
 }  // namespace
 
-// CG with a two-level DILU can apply M^{-1} inside its x/r phase by
-// recomputing neighbour values (2 instead of 3 grid barriers per iteration,
-// identical results).  On B200 the extra chain of dependent L2 gathers costs
-// more than the barrier it saves (47,385-cell BFS: 1.73 vs 1.48 ms per SIMPLE
-// iteration; 128^3 cavity: 44 vs 33 ms), so it is off unless XCAL_CG_FUSE=1.
-static int choose_cg_fuse(int ntiles, int nblocks) {
-  const char *f = getenv("XCAL_CG_FUSE");
-  (void)ntiles; (void)nblocks;
-  return f ? atoi(f) != 0 : 0;
-}
-
 // Grid-barrier wait limit and expected extra arrivals, read on every run:
 // XCAL_BARRIER_TIMEOUT_US (default 2 s) bounds one wait; XCAL_BARRIER_EXTRA
 // (default 0) makes every wait expect that many arrivals beyond the launch's
@@ -234,7 +223,7 @@ struct TuneKey {
   }
 };
 struct TuneChoice {
-  int mode, occ, nblocks, cg_fuse;
+  int mode, occ, nblocks;
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneChoice> g_tune;
@@ -246,14 +235,9 @@ static TuneKey tune_key(xcal_ctx c, int prec) {
   return TuneKey{c->ns, b, c->prep.W, prec};
 }
 
-static void choose_launch(xcal_ctx c, int n, KParams &h) {
-  choose_launch_mode(c, n);
-  h.cg_fuse = choose_cg_fuse((n + TILE - 1) / TILE, c->nblocks);
-}
-
 // A tuned form for this context's class, unless the environment forces one.
 static void apply_tuned(xcal_ctx c, int prec) {
-  if (getenv("XCAL_SYNC") || getenv("XCAL_OCC") || getenv("XCAL_NBLOCKS") || getenv("XCAL_CG_FUSE")) return;
+  if (getenv("XCAL_SYNC") || getenv("XCAL_OCC") || getenv("XCAL_NBLOCKS")) return;
   if (c->flags & XCAL_FLAG_CLUSTER) return;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tune.find(tune_key(c, prec));
@@ -261,7 +245,6 @@ static void apply_tuned(xcal_ctx c, int prec) {
   c->mode = it->second.mode;
   c->occ = it->second.occ;
   c->nblocks = it->second.nblocks;
-  c->hp.cg_fuse = it->second.cg_fuse;
 }
 
 // Build of the persistent program for a grid launch: the 4-CTA/SM build once
@@ -555,6 +538,12 @@ static int mesh_arrays(xcal_ctx c, Sink &S) {
   h.f_sign = S.put_v(P.f_sign); h.f_first = S.put_v(P.f_first);
   h.cb_ptr = S.put_v(P.cb_ptr); h.cb_face = S.put_v(P.cb_face);
   h.flev = S.put_v(P.flev); h.blev = S.put_v(P.blev);
+  h.sweep = -1;
+  if (!P.lists.frow.empty()) {
+    h.sweep = 0;
+    h.frow = S.put_v(P.lists.frow); h.brow = S.put_v(P.lists.brow);
+    h.items = S.put_v(P.lists.items); h.lptr = S.put_v(P.lists.ptr);
+  }
   const int *ecol = S.put_v(P.e_col), *etpos = S.put_v(P.e_tpos), *edpos = S.put_v(P.dpos);
   for (Mat *A : {&h.AU, &h.AP}) { A->col = ecol; A->tpos = etpos; A->dpos = edpos; A->W = P.W; A->np = P.np; }
   if (!S.ok()) return fail(c, S.error(), S.message());
@@ -576,7 +565,7 @@ int xcal_mesh_upload(xcal_ctx c, const xcal_mesh_desc *d, int32_t renumber) {
   TRY(mesh_prepare(c, d, renumber));
   DevSink S(c, c->mbuf);
   TRY(mesh_arrays(c, S));
-  choose_launch(c, c->prep.n, c->hp);
+  choose_launch_mode(c, c->prep.n);
   {
     std::vector<int> p32(c->perm.begin(), c->perm.end());
     c->d_perm = S.put_v(p32);
@@ -981,7 +970,12 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   CUDA_TRY(c, cudaMemsetAsync(h.bar, 0, sizeof(Bar), c->stream));
   CUDA_TRY(c, cudaMemsetAsync(h.done, 0, sizeof(int), c->stream));
   h.mode = c->mode;
-  h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, c->occ, h.ntiles, c->nblocks);
+  // matrix rows in shared memory only for the solve that uses them: what it
+  // takes is lost to L1 (cavity 64^3, BiCGSTAB for p: 3.7 -> 4.1 ms)
+  h.ring = h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU
+               ? ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, c->occ, h.ntiles, c->nblocks)
+               : 0;
+  if (h.sweep >= 0) h.sweep = sweep_bytes((size_t)h.n * c->ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), c->occ);
   h.conv = c->conv;
   h.abort_nan = (c->flags & XCAL_FLAG_ABORT_ON_NAN) ? 1 : 0;
   barrier_knobs(h);
@@ -1005,7 +999,7 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   const int cgb = own && cluster.ctas == 0 && c->mode == SYNC_GRID && h.ring == 0 ? std::min(c->cg_ctas, h.ntiles) : 0;
   if (cluster.ctas > 0 || cgb > 0) {
     CUDA_TRY(c, cudaMemsetAsync(h.step, 0, sizeof(StepState), c->stream));
-    h.ring = 0;   // the program's launches hold no matrix rows
+    h.ring = 0;   // the program's launches hold no matrix rows (a two-level numbering has no sweeps by one CTA)
     const int total = iters * (prog == PROG_PISO ? 2 : 1);
     for (int k = 0; k <= total; ++k) {
       CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, k, c->stream));
@@ -1090,27 +1084,25 @@ int xcal_autotune(xcal_ctx c, int32_t iters, xcal_tune_result *out) {
   const bool gmres = h.wU.gmax > 0 || h.wP.gmax > 0;
   const int setup_ctas = c->nblocks;   // GMRES per-CTA scratch was sized for this many CTAs
   struct Cand {
-    int mode, occ, nblocks, cg_fuse;
+    int mode, occ, nblocks;
   };
   std::vector<Cand> cands;
-  cands.push_back({c->mode, c->occ, c->nblocks, h.cg_fuse});   // the heuristic's form first
-  auto add = [&](int mode, int occ, int nb, int fuse) {
+  cands.push_back({c->mode, c->occ, c->nblocks});   // the heuristic's form first
+  auto add = [&](int mode, int occ, int nb) {
     nb = std::max(1, nb);
     if (gmres && nb > setup_ctas) return;
     for (const Cand &k : cands)
-      if (k.mode == mode && k.occ == occ && k.nblocks == nb && k.cg_fuse == fuse) return;
-    cands.push_back({mode, occ, nb, fuse});
+      if (k.mode == mode && k.occ == occ && k.nblocks == nb) return;
+    cands.push_back({mode, occ, nb});
   };
   for (int occ = 0; occ <= (NS >= 2 ? 1 : 0); ++occ) {
     const int maxco = max_coresident_blocks(NS, occ, c->device);
     if (maxco < 1) continue;
-    add(SYNC_GRID, occ, std::min(maxco, ntiles), 0);
-    add(SYNC_GRID, occ, std::min(maxco / 2, ntiles), 0);
+    add(SYNC_GRID, occ, std::min(maxco, ntiles));
+    add(SYNC_GRID, occ, std::min(maxco / 2, ntiles));
   }
   const int mc = max_cluster_blocks(NS, 0);
-  if (ntiles <= mc) add(SYNC_CLUSTER, 0, ntiles, 0);
-  if (h.kP.solver == XCAL_SOLVER_CG && h.AP.precon == XCAL_PRECON_DILU && h.nfl == 2)
-    add(cands[0].mode, cands[0].occ, cands[0].nblocks, 1 - cands[0].cg_fuse);
+  if (ntiles <= mc) add(SYNC_CLUSTER, 0, ntiles);
   // fields the runs change, restored before every candidate and at the end
   DevBuf B;
   B.stream = c->stream;
@@ -1142,7 +1134,6 @@ int xcal_autotune(xcal_ctx c, int32_t iters, xcal_tune_result *out) {
     c->mode = cands[k].mode;
     c->occ = cands[k].occ;
     c->nblocks = cands[k].nblocks;
-    h.cg_fuse = cands[k].cg_fuse;
     st = restore();
     if (st == XCAL_OK) st = run_program(c, PROG_SIMPLE, 1, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     if (st == XCAL_OK) st = restore();
@@ -1160,19 +1151,18 @@ int xcal_autotune(xcal_ctx c, int32_t iters, xcal_tune_result *out) {
   c->mode = b.mode;
   c->occ = b.occ;
   c->nblocks = b.nblocks;
-  h.cg_fuse = b.cg_fuse;
   const int rs = restore();
   if (st != XCAL_OK) return st;
   TRY(rs);
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[tune_key(c, h.prec)] = TuneChoice{b.mode, b.occ, b.nblocks, b.cg_fuse};
+    g_tune[tune_key(c, h.prec)] = TuneChoice{b.mode, b.occ, b.nblocks};
   }
   out->mode = b.mode;
   out->ctas = b.nblocks;
   out->ctas_per_sm = b.occ ? 4 : 2;
-  out->cg_fused = b.cg_fuse;
+  out->cg_fused = 0;
   out->candidates = (int32_t)cands.size();
   out->ms_per_iteration = best;
   out->ms_default = first;
@@ -1290,6 +1280,13 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
   TRY(upload_c(c, B, h.flev, fl)); TRY(upload_c(c, B, h.blev, bl));
   h.nfl = nfl; h.nbl = nbl;
   h.n0 = two_level_rows(fl, n, nfl, nbl);
+  const LevelLists lists = level_lists(fl, bl, n, nfl, nbl);
+  h.sweep = -1;
+  if (!lists.frow.empty()) {
+    h.sweep = sweep_bytes((size_t)n * sizeof(double), 0);
+    TRY(upload_c(c, B, h.frow, lists.frow)); TRY(upload_c(c, B, h.brow, lists.brow));
+    TRY(upload_c(c, B, h.items, lists.items)); TRY(upload_c(c, B, h.lptr, lists.ptr));
+  }
   TRY(upload_c(c, B, h.AU.col, ecol)); TRY(upload_c(c, B, h.AU.tpos, etp)); TRY(upload_c(c, B, h.AU.dpos, edp));
   h.AU.W = W; h.AU.np = np;
   std::vector<double> bb(b, b + n), xx(x, x + n);
@@ -1315,12 +1312,12 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
   {
     int saved_ns = c->ns, saved_mode = c->mode, saved_nb = c->nblocks, saved_occ = c->occ;
     c->ns = 1;
-    choose_launch(c, n, h);
+    choose_launch_mode(c, n);
     mode = c->mode; nb = c->nblocks;
     c->ns = saved_ns; c->mode = saved_mode; c->nblocks = saved_nb; c->occ = saved_occ;
   }
   h.mode = mode;
-  h.ring = ring_tiles(W, 0, 0, h.ntiles, nb);
+  h.ring = h.n0 > 0 && solver == XCAL_SOLVER_CG && precon == XCAL_PRECON_DILU ? ring_tiles(W, 0, 0, h.ntiles, nb) : 0;
   if (solver == XCAL_SOLVER_GMRES) {
     double *g1 = nullptr, *g2 = nullptr;
     std::function<double *(size_t)> allocD = [&](size_t cnt) { return A(cnt); };
@@ -1768,7 +1765,7 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
   h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, gmres_ctas);   // the serving build: 4 CTAs per SM
-  h.cg_fuse = 0;
+  if (h.sweep >= 0) h.sweep = sweep_bytes((size_t)h.n * c.ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 1);
   h.phase = nullptr;
   h.bar = nullptr;   // the serving loop gives the case a barrier word when it starts
   out.prm = h;

@@ -78,9 +78,14 @@ struct MatT {
 };
 using Mat = MatT<double>;
 
-// CG in one cluster (xcal_cg_cluster_kernel): threads and vectors per CTA,
+// CG in one cluster (xcal_cg_cluster_kernel): most threads of a CTA, vectors,
 // most tiles of the mesh (one partial per lane of the final sum) and of a CTA.
-constexpr int CGC_TPB = 1024, CGC_VECTORS = 8, CGC_TILES = 256, CGC_SLOTS = 16;
+// At 8 tiles a CTA makes two rounds of a phase; with more the resident form in
+// the program is as fast or faster (ms per SIMPLE iteration, cluster / program:
+// cavity 128^2 0.757 / 1.034, 164^2 0.982 / 1.059, 164^2 mixed 0.912 / 1.063,
+// 200^2 mixed, 10 tiles, 1.160 / 1.084; hex 28^3 0.705 / 0.778, 35^3 mixed, 11
+// tiles, 0.731 / 0.770).
+constexpr int CGC_TPB = 1024, CGC_VECTORS = 8, CGC_TILES = 256, CGC_SLOTS = 8;
 // Tiles of a group (count N) given to CTA b of G: [chunk(b), chunk(b+1)).
 __host__ __device__ inline int chunk(int b, int N, int G) { return (int)((long long)b * N / G); }
 
@@ -118,7 +123,13 @@ struct KParams {
   int nfl, nbl;
   int n0;          // rows [0, n0) of DILU level 0 and [n0, n) of level 1, all of them (0: any other numbering)
   int ring;        // matrix tiles the launch's dynamic shared memory holds (row width W, the Krylov value type)
-  int cg_fuse;     // CG: M^{-1} of a two-level DILU inside the x/r phase (2 barriers per iteration)
+  // sweeps by one CTA (many narrow levels): bytes of dynamic shared memory
+  // (-1: level by level over the grid); rows listed by forward and by backward
+  // level; items of up to 32 rows of a level (first row, end), forward then
+  // backward; the first item of each level
+  // (nfl+1, then nbl+1 values)
+  int sweep;
+  const int *frow, *brow, *items, *lptr;
   int abort_nan;   // stop at the first non-finite Krylov residual norm
   double conv;     // SIMPLE stop: every residual <= conv (1e-7 in the reference)
   Mat AU, AP;

@@ -61,9 +61,13 @@ __device__ __forceinline__ void lev_bwd_row(const MatT<T> &A, const T *out, int 
 // into registers instead of reaching through a pointer for each of them.
 struct Ctx {
   const KParams *P;
-  int n, np, ntiles, nfl, nbl, cg_fuse;
+  int n, np, ntiles, nfl, nbl;
   int n0, ring;   // rows of level 0 of a two-level numbering (0: other numberings); matrix tiles the dynamic shared memory holds
   const int *flev, *blev;
+  // sweeps by one CTA: bytes of dynamic shared memory for the vector (-1: the
+  // grid's CTAs sweep level by level), the rows listed level by level, items
+  int sweep;
+  const int *frow, *brow, *items, *lptr;
   int copies;     // rounds of bulk copies done (the parity of their barrier)
   Sync S;
   // Per-tile partial sums, two buffers of MAXK*ntiles used in turn by
@@ -123,10 +127,16 @@ __device__ __forceinline__ void ctx_mesh(Ctx &C, const KParams &P) {
   C.ntiles = P.ntiles;
   C.nfl = P.nfl;
   C.nbl = P.nbl;
-  C.cg_fuse = P.cg_fuse;
   C.n0 = P.n0;
   C.ring = P.ring;
   C.copies = 0;
+  C.sweep = P.sweep;
+  C.frow = P.frow;
+  C.brow = P.brow;
+  C.items = P.items;
+  C.lptr = P.lptr;
+  C.flev = P.flev;
+  C.blev = P.blev;
 }
 
 template <typename T>
@@ -341,6 +351,163 @@ __device__ __forceinline__ bool precon_local(const PT &P, const MatT<T> &A, int 
   return true;
 }
 
+// The sweeps of a numbering with many narrow levels (the caller's own order,
+// RCM: a level is a wavefront of a few dozen rows) by one CTA.  A barrier over
+// the grid per level costs about 3.5 us whatever the level holds.  Here a level
+// is cut into items of up to 32 rows, dealt to the CTA's warps in turn: a warp
+// fetches the entries of its next item, a chain of dependent loads that the
+// solution is no part of, while the other warps pass the levels between, and
+// then works on the vector, which is in shared memory where it fits, when the
+// block barrier of the level before is passed.  The other CTAs wait at the
+// barrier that ends the sweeps.  Row arithmetic is that of the row routines.
+// (A count of the items done, polled by the warps, in place of the block
+// barrier: its release waits for the fetches in flight, 1.4 us per level.)
+extern __shared__ __align__(128) unsigned char s_dyn[];
+
+struct SweepArgs {   // what the sweeps need of Ctx, by value: they are called out of line
+  int n, nfl, nbl, sweep;
+  const int *blev, *frow, *brow, *items, *lptr;
+};
+
+// One row's entries on one side of the diagonal: for DILU forward the lower
+// ones with their Dinv, backward the upper ones.
+template <typename T, int WS>
+struct SweepRow {
+  int i;        // -1: none
+  int last;     // forward: the row has no upper neighbours
+  int c[WS];    // neighbour, -1: not on this side
+  T a[WS], d[WS], di;
+};
+template <bool FWD, typename T, int WS>
+__device__ __forceinline__ void sweep_load(const SweepArgs &C, const MatT<T> &A, int i, SweepRow<T, WS> &r) {
+  r.i = i;
+  const int ii = max(i, 0);
+  r.di = A.Dinv[ii];
+  r.last = FWD ? ldro(C.blev + ii) == 0 : 0;
+#pragma unroll
+  for (int k = 0; k < WS; ++k) {
+    const int kk = k < A.W ? k : A.W - 1;
+    const int c = (i >= 0 && k < A.W) ? ldro(A.col + (size_t)kk * A.np + ii) : -1;
+    const bool use = FWD ? (c >= 0 && c < ii) : c > ii;
+    r.c[k] = use ? c : -1;
+    r.a[k] = A.val[(size_t)kk * A.np + ii];
+    r.d[k] = FWD ? A.Dinv[use ? c : ii] : T(0);
+  }
+}
+
+template <int NS, bool FWD, typename T, int WS>
+__device__ __forceinline__ void sweep_row(const SweepRow<T, WS> &r, const T *in, T *x) {
+  if (r.i < 0) return;
+#pragma unroll
+  for (int d = 0; d < NS; ++d) {
+    T o = FWD ? in[(size_t)r.i * NS + d] : x[(size_t)r.i * NS + d] * r.di;
+#pragma unroll
+    for (int k = 0; k < WS; ++k) {
+      const int j = r.c[k] >= 0 ? r.c[k] : r.i;
+      const T t = o - r.a[k] * x[(size_t)j * NS + d] * (FWD ? r.d[k] : r.di);
+      o = r.c[k] >= 0 ? t : o;
+    }
+    if (FWD && r.last) o = o * r.di;
+    x[(size_t)r.i * NS + d] = o;
+  }
+}
+
+// Levels first.. of one direction.  Item q is rows[item[2q]..item[2q+1]) of one
+// level; ptr[l] is the first item of level l, ptr[nlev] their number.  x is the
+// vector solved for (out in global memory or its copy in shared memory), in
+// the right-hand side of the forward sweep.
+template <int NS, bool FWD, typename T, int WS>
+__device__ __forceinline__ void sweep_levels(const SweepArgs &C, const MatT<T> &A, const int *rows, const int *item,
+                                             const int *ptr, int first, int nlev, const T *in, T *x) {
+  constexpr int NW = TPB / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int q0 = ldro(ptr + first), nq = ldro(ptr + nlev);
+  auto row_of = [&](int q) {
+    const int p = ldro(item + 2 * q) + lane;
+    return p < ldro(item + 2 * q + 1) ? ldro(rows + p) : -1;
+  };
+  // own items q, q + NW, ...: the entries of the next one and the row of the
+  // one after it are on their way.  Two buffers used in turn, not one copied
+  // into the other: a copy would wait for the loads.
+  SweepRow<T, WS> r0, r1;
+  int q = q0 + wid, inext = -1;
+  bool odd = false;
+  if (q < nq) sweep_load<FWD>(C, A, row_of(q), r0);
+  if (q + NW < nq) inext = row_of(q + NW);
+  int end = ldro(ptr + first + 1);
+  for (int l = first; l < nlev; ++l) {
+    const int end_next = ldro(ptr + min(l + 2, nlev));
+    for (; q < end; q += NW) {
+      if (odd) {
+        if (q + NW < nq) sweep_load<FWD>(C, A, inext, r0);
+        sweep_row<NS, FWD>(r1, in, x);
+      } else {
+        if (q + NW < nq) sweep_load<FWD>(C, A, inext, r1);
+        sweep_row<NS, FWD>(r0, in, x);
+      }
+      odd = !odd;
+      if (q + 2 * NW < nq) inext = row_of(q + 2 * NW);
+    }
+    __syncthreads();
+    end = end_next;
+  }
+}
+
+template <int NS, typename T, int WS>
+__device__ __forceinline__ void sweep_both(const SweepArgs &C, const MatT<T> &A, const int *fitem, const int *bitem,
+                                           int first, const T *in, T *x) {
+  const int *fptr = C.lptr, *bptr = C.lptr + C.nfl + 1;
+  if (first < C.nfl) sweep_levels<NS, true, T, WS>(C, A, C.frow, fitem, fptr, first, C.nfl, in, x);
+  if (C.nbl > 1) sweep_levels<NS, false, T, WS>(C, A, C.brow, bitem, bptr, 1, C.nbl, in, x);
+}
+
+template <int NS, typename T>
+__device__ __noinline__ void sweep_by_one(SweepArgs C, MatT<T> A, const T *in, T *out, bool setup, int first) {
+  const int tid = threadIdx.x, len = C.n * NS;
+  const int *fptr = C.lptr, *bptr = C.lptr + C.nfl + 1;
+  const int *fitem = C.items, *bitem = C.items + 2 * ldro(fptr + C.nfl);
+  if (setup || A.precon != PRECON_DILU || A.W > WUNROLL) {
+    // pivots on the way, or ILU(0) rows: level by level, nothing fetched
+    // ahead, the vector in global memory
+    for (int l = first; l < C.nfl; ++l) {
+      const int end = ldro(fitem + 2 * (ldro(fptr + l + 1) - 1) + 1);
+      for (int p = ldro(fitem + 2 * ldro(fptr + l)) + tid; p < end; p += TPB) {
+        const int i = ldro(C.frow + p);
+        if (setup) lev_setup_row(A, i);
+        T iv[NS], o[NS];
+#pragma unroll
+        for (int d = 0; d < NS; ++d) iv[d] = in[(size_t)i * NS + d];
+        lev_fwd_row<NS>(A, iv, [&](int j, int d) { return out[(size_t)j * NS + d]; }, i, ldro(C.blev + i), o);
+#pragma unroll
+        for (int d = 0; d < NS; ++d) out[(size_t)i * NS + d] = o[d];
+      }
+      __syncthreads();
+    }
+    for (int l = 1; l < C.nbl; ++l) {
+      const int end = ldro(bitem + 2 * (ldro(bptr + l + 1) - 1) + 1);
+      for (int p = ldro(bitem + 2 * ldro(bptr + l)) + tid; p < end; p += TPB) {
+        const int i = ldro(C.brow + p);
+        T o[NS];
+        lev_bwd_row<NS>(A, out, i, o);
+#pragma unroll
+        for (int d = 0; d < NS; ++d) out[(size_t)i * NS + d] = o[d];
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const bool local = (size_t)len * sizeof(T) <= (size_t)C.sweep;
+  T *x = local ? (T *)s_dyn : out;
+  if (local) {   // rows below `first` were done by the phase before
+    for (int q = tid; q < len; q += TPB) x[q] = out[q];
+    __syncthreads();
+  }
+  if (A.W <= 5) sweep_both<NS, T, 5>(C, A, fitem, bitem, first, in, x);
+  else sweep_both<NS, T, WUNROLL>(C, A, fitem, bitem, first, in, x);
+  if (local)
+    for (int q = tid; q < len; q += TPB) out[q] = x[q];
+}
+
 // Number of phases of M^{-1} after its producer phase.  The producer did the
 // row-local part (and, with first_lvl == 2, forward level 1 as well).
 template <typename T>
@@ -352,11 +519,26 @@ __device__ __forceinline__ int precon_tail_phases(const Ctx &P, const MatT<T> &A
 // The remaining phases of M^{-1} (in -> out).  With `setup` the DILU pivots
 // (update_preconditioner!) are computed level by level in the same phases.
 // The last phase also computes the K partial sums red(i, v).
-template <int NS, int K, typename T, class Red, int R = 1>
+// ONE: with the sweeps by one CTA for the numberings that have them.
+template <int NS, int K, bool ONE, typename T, class Red, int R = 1>
 __device__ __forceinline__ bool precon_tail(Ctx &C, const MatT<T> &A, const T *in, T *out, bool setup, int first_lvl, Red red) {
   const Ctx &P = C;
   const int nph = precon_tail_phases(P, A, setup, first_lvl);
   C.phase(setup ? PH_PREC_SETUP : PH_KRY_PREC);
+  bool applied = nph == 0 && setup;   // nothing left to apply: reduce in a phase of its own
+  if constexpr (ONE) {
+    if (C.sweep >= 0 && leveled(A)) {
+      if (vbid() == 0)
+        sweep_by_one<NS, T>(SweepArgs{C.n, C.nfl, C.nbl, C.sweep, C.blev, C.frow, C.brow, C.items, C.lptr}, A, in, out,
+                            setup, first_lvl);
+      if (!C.sync()) return false;
+      applied = true;
+    }
+  }
+  if (applied) {
+    tile_phase<K>(C, true, [&](int i, double (&v)[K]) { red(i, v); });
+    return C.sync();
+  }
   if constexpr (R > 1) {
     if (!setup && A.precon == PRECON_DILU && nph > 0 && pairs_pay(P)) {
       // the DILU levels R rows at a time; in a warp holding a row of the
@@ -423,10 +605,6 @@ __device__ __forceinline__ bool precon_tail(Ctx &C, const MatT<T> &A, const T *i
       }
       return true;
     }
-  }
-  if (nph == 0 && setup) {   // nothing left to apply: reduce in a phase of its own
-    tile_phase<K>(C, true, [&](int i, double (&v)[K]) { red(i, v); });
-    return C.sync();
   }
   if (!leveled(A)) {
     if (!setup) return true;
@@ -519,10 +697,10 @@ __device__ __forceinline__ void krylov_init_row(const KParams &P, const Mat &A64
 // Set-up phases of M and its first application after the assembly phase,
 // with the initial dot products (CG: <r,z>; BiCGSTAB: <b,r>, <r,r>), all
 // accumulated in FP64.
-template <int NS, typename T>
-__device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, int solver) {
+template <int NS, bool ONE, typename T>
+__device__ __forceinline__ bool krylov_start_inl(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, int solver) {
   if (solver != SOLVER_CG) {
-    return precon_tail<NS, 2 * NS>(C, A, w.q, w.r[0], true, 1, [&](int i, double (&v)[2 * NS]) {
+    return precon_tail<NS, 2 * NS, ONE>(C, A, w.q, w.r[0], true, 1, [&](int i, double (&v)[2 * NS]) {
 #pragma unroll
       for (int d = 0; d < NS; ++d) {
         const double rv = (double)w.r[0][(size_t)i * NS + d];
@@ -531,11 +709,33 @@ __device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWo
       }
     });
   }
-  return precon_tail<NS, NS>(C, A, w.r[0], w.v[0], true, 1, [&](int i, double (&v)[NS]) {
+  return precon_tail<NS, NS, ONE>(C, A, w.r[0], w.v[0], true, 1, [&](int i, double (&v)[NS]) {
 #pragma unroll
     for (int d = 0; d < NS; ++d)
       v[d] = (double)w.r[0][(size_t)i * NS + d] * (double)w.v[0][(size_t)i * NS + d];
   });
+}
+
+// A call inside the program costs its callers registers, so the numberings
+// with sweeps by one CTA have their own, out-of-line start, as they have the
+// out-of-line solvers.
+template <int NS, typename T>
+__device__ __noinline__ bool krylov_start_one(Ctx *state, MatT<T> A, KWorkT<T> w, const double *b, int solver) {
+  Ctx C = *state;
+  const bool ok = krylov_start_inl<NS, true, T>(C, A, w, b, solver);
+  *state = C;
+  return ok;
+}
+template <int NS, typename T>
+__device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, int solver) {
+  if (C.sweep < 0) return krylov_start_inl<NS, false, T>(C, A, w, b, solver);
+  const KParams *P = C.P;
+  Ctx t = C;
+  t.P = nullptr;
+  const bool ok = krylov_start_one<NS, T>(&t, A, w, b, solver);
+  C = t;
+  C.P = P;
+  return ok;
 }
 
 // ------------------------------------------------------------- BiCGSTAB
@@ -548,7 +748,7 @@ __device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWo
 //   .. remaining M^-1 phases, last one reduces <t,s>, <t,t>
 //   G  x += omega*s, r = s - omega*t, reduces <b,r>, <r,r>
 // Vector updates are evaluated in FP64 and stored in T; dots accumulate in FP64.
-template <int NS, typename T>
+template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *bb, const KCfg &cfg,
                          int (&its)[NS], double (&rnorm_out)[NS]) {
   const Ctx &P = C;
@@ -604,7 +804,7 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
         for (int d = 0; d < NS; ++d) v[d] = bb[(size_t)i * NS + d] * (double)o[d];
     });
     if (!C.sync()) return false;
-    if (!precon_tail<NS, NS>(C, A, (const T *)w.q, vn, false, 1, [&](int i, double (&v)[NS]) {
+    if (!precon_tail<NS, NS, ONE>(C, A, (const T *)w.q, vn, false, 1, [&](int i, double (&v)[NS]) {
 #pragma unroll
           for (int d = 0; d < NS; ++d) v[d] = bb[(size_t)i * NS + d] * (double)vn[(size_t)i * NS + d];
         }))
@@ -647,7 +847,7 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
         }
     });
     if (!C.sync()) return false;
-    if (!precon_tail<NS, 2 * NS>(C, A, (const T *)w.q, w.t, false, 1, [&](int i, double (&v)[2 * NS]) {
+    if (!precon_tail<NS, 2 * NS, ONE>(C, A, (const T *)w.q, w.t, false, 1, [&](int i, double (&v)[2 * NS]) {
 #pragma unroll
           for (int d = 0; d < NS; ++d) {
             const size_t k = (size_t)i * NS + d;
@@ -719,7 +919,6 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
 // there: after a barrier, which empties L1, the columns come from shared
 // memory at once and the phase is one round of gathers long instead of two.
 // Otherwise the rows are read from global memory in every phase.
-extern __shared__ __align__(128) unsigned char s_dyn[];
 __shared__ unsigned long long s_full;   // mbarrier: the matrix tiles have arrived
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -995,7 +1194,7 @@ __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWo
 //   B  x += alpha p, r -= alpha q, M^-1 levels 0 and 1 (level-0 values of
 //      neighbours recomputed), backward step of rows without upper neighbours
 //   .. remaining M^-1 phases, the last reduces <r,z>
-template <int NS, typename T>
+template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                    double (&rnorm_out)[NS]) {
   const Ctx &P = C;
@@ -1020,13 +1219,7 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
   T *zw = w.v[0];
   const bool dilu = leveled(A);
   const bool lvl1 = dilu && P.nfl >= 2;
-  // With two forward levels every level-1 row has only lower neighbours and
-  // every level-0 row only upper ones, so the whole of M^{-1} r fits in the
-  // x/r phase: level-0 rows recompute their upper neighbours' forward values
-  // (which in turn recompute r of their level-0 neighbours).  Same row
-  // functions, same inputs: identical bits, one grid barrier fewer.
-  const bool fuse = A.precon == PRECON_DILU && P.nfl == 2 && P.cg_fuse;
-  const int tail = (dilu && !fuse) ? precon_tail_phases(P, A, false, 2) : 0;
+  const int tail = dilu ? precon_tail_phases(P, A, false, 2) : 0;
   int rc = 0, pc = 0;
   bool first = true;
   while (active) {
@@ -1090,7 +1283,7 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
     // B: x, r updates and M^{-1} levels 0/1
     C.phase(PH_KRY_PREC);
     if (CgRows<T>::R > 1 && pairs_pay(P)) {
-      if (A.precon == PRECON_DILU && !fuse) {
+      if (A.precon == PRECON_DILU) {
         // R rows at a time; a DILU row of level 0 or 1 is one forward row
         // (level 0: no lower neighbours, then its diagonal step when it has
         // no upper ones), the row-local part of precon_local for level 0
@@ -1160,28 +1353,10 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
         }
       }
       bool have;
-      if (fuse) {
-        if (ldro(P.flev + i) == 1) {
-          dilu_fwd_row<NS>(A, rr, getr, i, 0, o);
-        } else if (ldro(P.blev + i) == 0) {
-#pragma unroll
-          for (int d = 0; d < NS; ++d) o[d] = rr[d] * A.Dinv[i];
-        } else {
-          dilu_bwd_row_g<NS>(A, rr, [&](int j, int d) -> T {
-            T rj[NS], zj[NS];
-#pragma unroll
-            for (int e = 0; e < NS; ++e) rj[e] = getr(j, e);
-            dilu_fwd_row<NS>(A, rj, getr, j, 0, zj);
-            return zj[d];
-          }, i, o);
-        }
+      have = precon_local<NS>(P, A, i, rr, o);
+      if (!have && lvl1 && ldro(P.flev + i) == 1) {
+        lev_fwd_row<NS>(A, rr, getr, i, ldro(P.blev + i), o);
         have = true;
-      } else {
-        have = precon_local<NS>(P, A, i, rr, o);
-        if (!have && lvl1 && ldro(P.flev + i) == 1) {
-          lev_fwd_row<NS>(A, rr, getr, i, ldro(P.blev + i), o);
-          have = true;
-        }
       }
       if (have)
 #pragma unroll
@@ -1192,12 +1367,12 @@ __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w,
     });
   phase_b_done:
     if (!C.sync()) return false;
-    if (dilu && !fuse) {
+    if (dilu) {
       auto rz = [&](int i, double (&v)[NS]) {
 #pragma unroll
         for (int d = 0; d < NS; ++d) v[d] = (double)rn[(size_t)i * NS + d] * (double)z[(size_t)i * NS + d];
       };
-      if (!precon_tail<NS, NS, T, decltype(rz), CgRows<T>::R>(C, A, (const T *)rn, zw, false, 2, rz)) return false;
+      if (!precon_tail<NS, NS, ONE, T, decltype(rz), CgRows<T>::R>(C, A, (const T *)rn, zw, false, 2, rz)) return false;
     }
     final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
     unsigned cont = 0;
@@ -1265,7 +1440,7 @@ __device__ __forceinline__ void sym_givens(double a, double b, double &c, double
   }
 }
 
-template <int NS, typename T>
+template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                       double (&rnorm_out)[NS]) {
   const Ctx &P = C;
@@ -1330,7 +1505,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
         }
     });
     if (!C.sync()) return false;
-    if (!precon_tail<NS, NS>(C, A, (const T *)w.t, qn, false, 1, [&](int i, double (&v)[NS]) {
+    if (!precon_tail<NS, NS, ONE>(C, A, (const T *)w.t, qn, false, 1, [&](int i, double (&v)[NS]) {
 #pragma unroll
           for (int d = 0; d < NS; ++d)
             v[d] = (double)w.V[(size_t)i * NS + d] * (double)qn[(size_t)i * NS + d];
@@ -1445,20 +1620,21 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
   return true;
 }
 
-// The general solvers out of line, once per component count: inlined at each
-// call they made the program several times larger and its build minutes
-// longer.  The state and the operands are copied in (and the state back), so
-// the caller's own state stays in registers and the solver works on registers.
+// The general solvers out of line, once per component count.  The state is
+// copied in and back, so that the caller's own stays in registers; matrix and
+// vectors are read from shared memory (kept in registers they spilled).
+__shared__ __align__(16) unsigned char s_matrix[sizeof(Mat)], s_work[sizeof(KWork)];
 template <int NS, typename T>
-__device__ __noinline__ bool krylov_general(Ctx *state, MatT<T> A, KWorkT<T> w, const double *b, KCfg cfg, int *its,
-                                            double *rn) {
+__device__ __noinline__ bool krylov_general(Ctx *state, const double *b, KCfg cfg, int *its, double *rn) {
   Ctx C = *state;
+  const MatT<T> &A = *(const MatT<T> *)s_matrix;
+  const KWorkT<T> &w = *(const KWorkT<T> *)s_work;
   int it[NS];
   double r[NS];
   bool ok;
-  if (cfg.solver == SOLVER_BICGSTAB) ok = bicgstab<NS, T>(C, A, w, b, cfg, it, r);
-  else if (cfg.solver == SOLVER_GMRES) ok = gmres<NS, T>(C, A, w, cfg, it, r);
-  else ok = cg<NS, T>(C, A, w, cfg, it, r);
+  if (cfg.solver == SOLVER_BICGSTAB) ok = bicgstab<NS, true>(C, A, w, b, cfg, it, r);
+  else if (cfg.solver == SOLVER_GMRES) ok = gmres<NS, true>(C, A, w, cfg, it, r);
+  else ok = cg<NS, true>(C, A, w, cfg, it, r);
 #pragma unroll
   for (int d = 0; d < NS; ++d) {
     its[d] = it[d];
@@ -1470,34 +1646,44 @@ __device__ __noinline__ bool krylov_general(Ctx *state, MatT<T> A, KWorkT<T> w, 
 template <int NS, typename T>
 __device__ __forceinline__ bool krylov(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, const KCfg &cfg,
                                        int (&its)[NS], double (&rn)[NS]) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *(MatT<T> *)s_matrix = A;
+    *(KWorkT<T> *)s_work = w;
+  }
+  __syncthreads();
+  const KParams *P = C.P;
   Ctx t = C;
+  t.P = nullptr;   // were the parameters' address to leave the kernel, every read of them would go through memory
   int it[NS];
   double r[NS];
-  const bool ok = krylov_general<NS, T>(&t, A, w, b, cfg, it, r);
+  const bool ok = krylov_general<NS, T>(&t, b, cfg, it, r);
 #pragma unroll
   for (int d = 0; d < NS; ++d) {
     its[d] = it[d];
     rn[d] = r[d];
   }
   C = t;
+  C.P = P;
   return ok;
 }
 
-// Momentum solve: BiCGSTAB with DILU, the configurations' solver, inlined
-// (its operands are then the kernel's parameters).
+// Solves of the program: the solvers inlined, where their operands are the
+// kernel's parameters (out of line a phase costs up to 0.7 us more); for the
+// numberings with sweeps by one CTA, whose time is in the sweeps, and for CG
+// on a vector out of line.
 template <int NS, typename T>
 __device__ __forceinline__ bool solve_vector(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
                                              const KCfg &cfg, int (&its)[NS], double (&rn)[NS]) {
-  if (cfg.solver == SOLVER_BICGSTAB && A.precon == PRECON_DILU) return bicgstab<NS, T>(C, A, w, b, cfg, its, rn);
+  if (cfg.solver == SOLVER_BICGSTAB && C.sweep < 0) return bicgstab<NS, false>(C, A, w, b, cfg, its, rn);
+  if (cfg.solver == SOLVER_GMRES && C.sweep < 0) return gmres<NS, false>(C, A, w, cfg, its, rn);
   return krylov<NS, T>(C, A, w, b, cfg, its, rn);
 }
 
-// Scalar solve of a mesh of DIM dimensions: the two-level CG inlined here,
-// where its operands are the kernel's parameters, the general solvers out of
-// line.
+// Pressure solve of a mesh of DIM dimensions.
 template <int DIM, typename T>
-__device__ __forceinline__ bool solve_scalar(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
-                                             const KCfg &cfg, int (&its)[1], double (&rn)[1]) {
+__device__ __forceinline__ bool solve_pressure(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
+                                               const KCfg &cfg, int (&its)[1], double (&rn)[1]) {
   constexpr int WT = DIM == 2 ? 5 : DIM == 3 ? 7 : WUNROLL;   // rows of a quad or hex mesh
   if (cfg.solver == SOLVER_CG && A.precon == PRECON_DILU && C.n0 > 0 && A.W <= WUNROLL) {
     // (large meshes run the CG as a kernel of its own; here the rows of tiles
@@ -1511,9 +1697,8 @@ __device__ __forceinline__ bool solve_scalar(Ctx &C, const MatT<T> &A, const KWo
     if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, true>(C, A, w, cfg, its[0], rn[0]);
     return cg_two_level<T, WUNROLL, true>(C, A, w, cfg, its[0], rn[0]);
   }
-  if (DIM == 2 && cfg.solver == SOLVER_BICGSTAB && A.precon == PRECON_DILU)   // k and omega
-    return bicgstab<1, T>(C, A, w, b, cfg, its, rn);
-  return krylov<1, T>(C, A, w, b, cfg, its, rn);
+  if (cfg.solver == SOLVER_CG && C.sweep < 0) return cg<1, false>(C, A, w, cfg, its, rn);
+  return solve_vector<1, T>(C, A, w, b, cfg, its, rn);
 }
 
 // -------------------------------------------------------------- assembly
@@ -2012,7 +2197,7 @@ __device__ __forceinline__ bool turbulence(Ctx &C) {
     if (!krylov_start<1, T>(C, A, wk, P.bP, cfg.solver)) return false;
     int its[1];
     double rn[1];
-    if (!solve_scalar<NS, T>(C, A, wk, P.bP, cfg, its, rn)) return false;
+    if (!solve_vector<1, T>(C, A, wk, P.bP, cfg, its, rn)) return false;
     // run! copy-back, then constrain_boundary! for omega (:401-448)
     C.phase(PH_TURB);
     tile_each(C, [&](int i) {
@@ -2281,7 +2466,7 @@ __device__ __forceinline__ void simple_program(Ctx &C, int iters, bool piso, int
       if (vbid() == 0 && threadIdx.x == 0) P.step->pw = C.pw;
       return;
     }
-    if (!solve_scalar<NS, T>(C, matP<T>(P), workP<T>(P), P.bP, P.kP, its, rn)) return;
+    if (!solve_pressure<NS, T>(C, matP<T>(P), workP<T>(P), P.bP, P.kP, its, rn)) return;
   }
 }
 
@@ -2301,7 +2486,7 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
   cfg.rtol = P.solve_rtol;
   int its[1];
   double rn[1];
-  if (!solve_scalar<1, double>(C, P.AU, P.wU, P.sb, cfg, its, rn)) return;
+  if (!solve_pressure<1, double>(C, P.AU, P.wU, P.sb, cfg, its, rn)) return;
   tile_each(C, [&](int i) { P.U[i] = P.wU.x[i] + P.U[i]; });
   if (vbid() == 0 && threadIdx.x == 0) {
     P.solve_out[0] = (double)its[0];
@@ -2384,8 +2569,9 @@ __global__ void __launch_bounds__(TPB, MB) xcal_cg_kernel(const __grid_constant_
 //
 // A CTA holds a chunk of the tiles with level-0 rows and the same chunk of
 // the others: its rows are close together in the mesh, so most neighbours
-// are its own, and all CTAs work in each phase.  Four tiles at a time, one
-// per 256 threads.
+// are its own, and all CTAs work in each phase.  Up to four tiles at a time,
+// one per 256 threads (threads for tiles that are not there slow the barriers
+// down: cavity 40^2 A 2.57 -> 2.28 us, B and C 1.64 -> 1.54).
 enum { CV_Z = 0, CV_P = 1, CV_R = 3, CV_Q = 5, CV_D = 6, CV_X = 7 };   // vectors (p and r twice)
 static_assert(CV_X + 1 == CGC_VECTORS, "vectors of a row");
 
@@ -2424,7 +2610,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
   const int n = prm.n, n0 = prm.n0, np = prm.np, nt = prm.ntiles;
   const int W = WT < WUNROLL ? WT : A.W;
   const int tid = threadIdx.x, lane = tid & 31, tl = tid >> 8, r = tid & 255, wt = (tid >> 5) & 7;
-  const int G = gridDim.x, b = blockIdx.x;
+  const int G = gridDim.x, b = blockIdx.x, groups = blockDim.x / TILE;
   // tiles [0, N0) hold level-0 rows, the rest only level-1 rows; tile N0-1 may hold both
   const int N0 = (n0 - 1) / TILE + 1, N1 = nt - N0;
   const int a0 = chunk(b, N0, G), k0 = chunk(b + 1, N0, G) - a0;                // own level-0 tiles: slots [0, k0)
@@ -2446,7 +2632,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
   };
   // rows into shared memory; entry k's neighbour as the address of its z in
   // the cluster, with bit 0 for the diagonal and bit 1 for padding
-  for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+  for (int s = tl; s < cnt; s += groups) {
     const int l = s * TILE + r, i = tile_of(s) * TILE + r;
     const bool on = i < n;
     vec[CV_Z * L + l] = on ? w.v[0][i] : T(0);
@@ -2470,7 +2656,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
   int par = 0;
   {
     const double *p0 = prm.part + (size_t)(prm.step->pw ^ 1) * MAXK * nt;
-    if (tid < nt) part[par][tid] = p0[tid];
+    for (int q = tid; q < nt; q += (int)blockDim.x) part[par][q] = p0[q];
   }
   cluster_sync();
   // canonical sum of the tiles' partials (final_sum's tree; one tile per lane)
@@ -2497,7 +2683,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
   // every own tile's sum to every CTA, then the barrier
   auto exchange = [&]() {
     __syncthreads();
-    for (int q = tid; q < cnt * G; q += CGC_TPB) {
+    for (int q = tid; q < cnt * G; q += (int)blockDim.x) {
       const int s = q / G;
       const double *ww = ws + s * 8;
       double x0 = ww[0] + ww[4], x1 = ww[1] + ww[5];
@@ -2526,7 +2712,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
     // A
     {
       const unsigned opo = (unsigned)(po * L * sizeof(T));
-      for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+      for (int s = tl; s < cnt; s += groups) {
         const int l = s * TILE + r;
         T y = T(0), pi = T(0), poi = T(0);
 #pragma unroll
@@ -2558,7 +2744,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
     const unsigned oro = (unsigned)(ro * L * sizeof(T)), oq = (unsigned)(CV_Q * L * sizeof(T)),
                    od = (unsigned)(CV_D * L * sizeof(T));
     // B
-    for (int s = sB + tl; s < cnt; s += CGC_TPB / TILE) {
+    for (int s = sB + tl; s < cnt; s += groups) {
       const int l = s * TILE + r, i = tile_of(s) * TILE + r;
       double rz = 0.0;
       if (i < n && i >= n0) {
@@ -2584,7 +2770,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
     cluster_sync();
     tick(1);
     // C
-    for (int s = tl; s < k0; s += CGC_TPB / TILE) {
+    for (int s = tl; s < k0; s += groups) {
       const int l = s * TILE + r, i = tile_of(s) * TILE + r;
       double rz = 0.0;
       if (i < n0) {
@@ -2630,7 +2816,7 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
     pspare = tp;
     po = tp;
   }
-  for (int s = tl; s < cnt; s += CGC_TPB / TILE) {
+  for (int s = tl; s < cnt; s += groups) {
     const int l = s * TILE + r, i = tile_of(s) * TILE + r;
     const T x = vec[CV_X * L + l];
     if (i < n) w.x[i] = pending ? vaxpy<T>(x, alpha, vec[po * L + l]) : x;

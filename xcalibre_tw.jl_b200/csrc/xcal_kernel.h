@@ -23,6 +23,9 @@ cudaError_t launch_cg_cluster(int mixed, const CgCluster &form, const KParams *h
 // Matrix tiles of the launch's dynamic shared memory ring (KParams::ring).
 int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks);
 size_t serve_dynamic_smem();
+// Dynamic shared memory for the vector of a sweep by one CTA (a vector that
+// does not fit stays in global memory).
+int sweep_bytes(size_t bytes, int occ);
 int max_coresident_blocks(int ns, int occ, int device);
 int max_cluster_blocks(int ns, int occ = 0);
 const void *program_kernel_ptr(int ns, int mixed, int occ);

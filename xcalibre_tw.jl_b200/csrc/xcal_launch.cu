@@ -46,6 +46,8 @@ int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks) {
   return want <= cap ? want : 0;
 }
 
+int sweep_bytes(size_t bytes, int occ) { return (int)std::min(bytes, RING_BYTES[occ ? 1 : 0]); }
+
 // Serving kernel of a dimension and precision (4-CTA/SM builds).
 const void *serve_kernel_ptr(int ns, int mixed) {
   if (ns == 2) return mixed ? serve_kernel_f2o() : serve_kernel_d2o();
@@ -111,7 +113,8 @@ cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, co
   args[0] = (void *)hparams;
   args[1] = (void *)&prog;
   args[2] = (void *)&iters;
-  const size_t dyn = hparams->ring * ring_tile_bytes(hparams->AU.W, mixed);   // one row width for both matrices
+  const size_t dyn = std::max(hparams->ring * ring_tile_bytes(hparams->AU.W, mixed),   // one row width for both matrices
+                              (size_t)std::max(hparams->sweep, 0));
   cudaError_t e = allow_ring(fn, occ);
   if (e != cudaSuccess) return e;
   if (mode == SYNC_BLOCK) return cudaLaunchKernel(fn, dim3(1), dim3(TPB), args, dyn, stream);
@@ -200,7 +203,7 @@ CgCluster cg_cluster(int mixed, int W, int n0, int ntiles) {
 cudaError_t launch_cg_cluster(int mixed, const CgCluster &form, const KParams *hparams, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(form.ctas);
-  cfg.blockDim = dim3(CGC_TPB);
+  cfg.blockDim = dim3(TILE * std::min(CGC_TPB / TILE, form.slots));
   cfg.dynamicSmemBytes = cgc_bytes(mixed, hparams->AP.W, form.slots);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
