@@ -47,6 +47,17 @@ UNIT = "cell-iters/s"
 RENUMBER = {"none": 0, "rcm": 1, "color": 2}
 
 
+def launches_per_step(cells, ns, renumber, precision):
+    """Kernels of one run(1): the program, or the program before and after the
+    pressure CG where that is a kernel of its own (two-colour numbering: small
+    meshes in one cluster, large ones beyond the program's shared memory)."""
+    tiles, width, size = -(-cells // 256), 7 if ns == 3 else 5, 4 if precision == "mixed" else 8
+    share = -(-tiles // 16)
+    cluster = share <= 8 and share * 256 * ((8 + width) * size + 4 * width) <= 220 * 1024
+    resident = tiles <= 148 * 4 * (48 * 1024 // (width * 256 * (size + 4)))
+    return 3 if renumber == "color" and (cluster or not resident) else 1
+
+
 def parse():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -718,7 +729,7 @@ def main():
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "steps": e2e_steps, "precision": main_name},
-        "gpu_launches": a.steps,
+        "gpu_launches": a.steps * launches_per_step(N, ns, a.renumber, main_name),
         "clocks": clocks,
         "impl": "xcal",
     }
