@@ -68,7 +68,6 @@ struct Ctx {
   // grid's CTAs sweep level by level), the rows listed level by level, items
   int sweep;
   const int *frow, *brow, *items, *lptr;
-  int copies;     // rounds of bulk copies done (the parity of their barrier)
   Sync S;
   // Per-tile partial sums, two buffers of MAXK*ntiles used in turn by
   // successive reducing phases.  A CTA reads a reduction's partials after the
@@ -103,8 +102,7 @@ struct Ctx {
   // (over one or more phases), then end_sum, which is a barrier of the whole
   // group and gives every thread the canonical sum.
   __device__ __forceinline__ void put_part(int t, double v) { part_w()[t] = v; }
-  __device__ __forceinline__ bool end_sum(double &out, bool ok) {
-    if (!ok) atomicExch(&S.bar->err, ST_TIMEOUT);   // the barrier then ends for every CTA
+  __device__ __forceinline__ bool end_sum(double &out) {
     pw ^= 1;
     if (!sync()) return false;
     double r[1];
@@ -129,7 +127,6 @@ __device__ __forceinline__ void ctx_mesh(Ctx &C, const KParams &P) {
   C.nbl = P.nbl;
   C.n0 = P.n0;
   C.ring = P.ring;
-  C.copies = 0;
   C.sweep = P.sweep;
   C.frow = P.frow;
   C.brow = P.brow;
@@ -914,60 +911,23 @@ __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<
 // A tile's <r, z> is summed in the phase that completes it.
 //
 // RES: the CTA's matrix tiles (values and columns) are copied into shared
-// memory at the start of the solve by bulk copies of one thread (the 256
-// entries of one row position are contiguous in the ELL layout) and stay
-// there: after a barrier, which empties L1, the columns come from shared
-// memory at once and the phase is one round of gathers long instead of two
-// (BFS 47k, one tile per CTA: A 4.1 -> 3.8 us, B and C 4.0 -> 2.8; the grid
-// barrier is 1.2 us of it, the sum of A and C 0.5).  Otherwise the rows are
-// read from global memory in every phase.
-__shared__ unsigned long long s_full;   // mbarrier: the matrix tiles have arrived
-
+// memory at the start of the solve (the 256 entries of one row position are
+// contiguous in the ELL layout) and stay there: after a barrier, which empties
+// L1, the columns come from shared memory at once and the phase is one round
+// of gathers long instead of two (BFS 47k, one tile per CTA: A 4.1 -> 3.6 us, B
+// and C 4.0 -> 2.7; the grid barrier is 1.2 us of it, the sum of A and C 0.5).
+// Otherwise the rows are read from global memory in every phase.
+//
+// The columns become addresses, so the rows are copied by each thread's own
+// asynchronous 16-byte copies, all in flight together, whose completion is
+// part of the instruction stream: there is no flag to wait for and no wait
+// that could run out with the columns unset.
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long *b, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+// 16 bytes into shared memory, through L2 (the matrix was written in this launch).
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void mbar_inval(unsigned long long *b) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(unsigned long long *b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for the phase of the given parity, at most limit_ns.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, unsigned long long limit_ns) {
-  if (mbar_try(b, parity)) return true;
-  const unsigned long long t = globaltimer();
-  while (!mbar_try(b, parity))
-    if (globaltimer() - t > limit_ns) return false;
-  return true;
-}
-// Copy of `bytes` (a multiple of 16; both addresses 16-byte aligned) into shared memory.
-__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, unsigned long long *b) {
-  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(b))
-               : "memory");
-}
-
-// The barrier of the copies, by the whole CTA at the start of a launch or of
-// a serving job (`again`: the barrier of the job before is given up).
-__device__ __forceinline__ void copies_init(bool again) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (again) mbar_inval(&s_full);
-    mbar_init(&s_full, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename T, int WT, bool RES>
 __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int &its_out,
@@ -984,22 +944,18 @@ __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWo
   const int m1 = t1 > B0 ? min(cnt, (t1 - B0 + G - 1) / G) : 0;   // with level-1 rows: m in [m1, cnt)
   T *sv = (T *)s_dyn;
   int *sc = (int *)(s_dyn + (size_t)C.ring * W * TILE * sizeof(T));
-  bool arrived = true;
   if (RES) {
-    if (tid == 0) {
-      // the matrix was written through ordinary stores, which this thread has
-      // acquired with the last barrier: order them before the bulk copies
-      asm volatile("fence.proxy.async;" ::: "memory");
-      mbar_expect(&s_full, cnt * W * TILE * (unsigned)(sizeof(T) + sizeof(int)));
-      for (int m = 0; m < cnt; ++m)
-        for (int k = 0; k < W; ++k) {
-          const size_t e = (size_t)k * np + (size_t)(B0 + G * m) * TILE;
-          bulk_copy(sv + (size_t)(m * W + k) * TILE, A.val + e, TILE * sizeof(T), &s_full);
-          bulk_copy(sc + (size_t)(m * W + k) * TILE, A.col + e, TILE * sizeof(int), &s_full);
-        }
-    }
-    arrived = mbar_wait(&s_full, C.copies & 1, C.S.timeout_ns);
-    C.copies += 1;
+    // one row position at a time: the first threads take its values, the next its columns
+    constexpr int V = 16 / sizeof(T), NV = TILE / V, NC = TILE / 4;
+    static_assert(NV + NC <= TPB, "one copy per thread and row position");
+    for (int m = 0; m < cnt; ++m)
+      for (int k = 0; k < W; ++k) {
+        const size_t g = (size_t)k * np + (size_t)(B0 + G * m) * TILE, l = (size_t)(m * W + k) * TILE;
+        if (tid < NV) copy16(sv + l + V * tid, A.val + g + V * tid);
+        else if (tid < NV + NC) copy16(sc + l + 4 * (tid - NV), A.col + g + 4 * (tid - NV));
+      }
+    copies_wait();
+    __syncthreads();
   }
   // first entry of row i of own tile m; entry k is at [k * ks]
   const size_t ks = RES ? (size_t)TILE : (size_t)np;
@@ -1085,7 +1041,7 @@ __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWo
     }
     pending = false;
     double s;
-    if (!C.end_sum(s, arrived)) return false;
+    if (!C.end_sum(s)) return false;
     const double pAp = sgn * s;
     if (pAp <= EPS * pn2 && fabs(pAp) <= EPS * pn2) break;   // zero curvature: stop
     alpha = gamma / pAp;
@@ -1156,7 +1112,7 @@ __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWo
         if (m > 0) __syncthreads();
       }
     }
-    if (!C.end_sum(s, arrived)) return false;
+    if (!C.end_sum(s)) return false;
     const double gn = sgn * s;
     rnorm = sqrt(gn);
     const bool solved = (rnorm <= eps) || (rnorm + 1.0 <= 1.0);
@@ -2502,7 +2458,6 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
 // State of a launch whose CTAs are all of one group.
 __device__ __forceinline__ void launch_begin(Ctx &C, const KParams &prm) {
   ctx_mesh(C, prm);
-  copies_init(false);
   C.S.bar = prm.bar;
   C.S.mode = prm.mode;
   C.S.nb = gridDim.x;
@@ -2892,7 +2847,6 @@ __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, co
   __shared__ int s_cmd;
   static_assert(sizeof(ServeJob) % 8 == 0, "job record copied in 8-byte words");
   ServeMail *m = mail + blockIdx.x;
-  unsigned jobs = 0;
   unsigned long long seen = 0;
   if (threadIdx.x == 0) seen = *(volatile unsigned long long *)&m->ack;
   for (;;) {
@@ -2959,7 +2913,6 @@ __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, co
     }
     Ctx C;
     ctx_mesh(C, sP);
-    copies_init(jobs++ > 0);
     C.S.bar = sP.bar;
     C.S.mode = SYNC_GRID;
     C.S.nb = G;
