@@ -553,9 +553,11 @@ void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reord
 LevelLists level_lists(const std::vector<int> &flev, const std::vector<int> &blev, int n, int nfl, int nbl) {
   LevelLists L;
   if ((nfl <= 2 && nbl <= 2) || n > (long long)SWEEP_WIDTH * std::min(nfl, nbl)) return L;
+  bool wide = false;
   auto list = [&](const std::vector<int> &lev, int nl, std::vector<int> &row) {
     std::vector<int> ptr(nl + 1, 0);
     for (int i = 0; i < n; ++i) ptr[lev[i] + 1]++;
+    wide = wide || *std::max_element(ptr.begin(), ptr.end()) > SWEEP_WIDEST;
     for (int l = 0; l < nl; ++l) ptr[l + 1] += ptr[l];
     int count = 0;
     for (int l = 0; l < nl; ++l) {
@@ -569,7 +571,7 @@ LevelLists level_lists(const std::vector<int> &flev, const std::vector<int> &ble
   };
   list(flev, nfl, L.frow);
   list(blev, nbl, L.brow);
-  return L;
+  return wide ? LevelLists{} : L;
 }
 
 int two_level_rows(const std::vector<int> &flev, int n, int nfl, int nbl) {

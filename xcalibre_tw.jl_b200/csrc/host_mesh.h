@@ -39,11 +39,13 @@ void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reord
 // Lists of the sweeps by one CTA (KParams::frow, brow, items, lptr): rows by
 // forward and by backward level, items of up to 32 rows of a level, the first
 // item of each level.  Empty where the grid sweeps level by level: two levels,
-// or levels of more than SWEEP_WIDTH rows on average.
+// levels of more than SWEEP_WIDTH rows on average, or any level of more than
+// SWEEP_WIDEST (64 rounds of the CTA's 256 threads, about 0.1 ms: the other CTAs
+// wait meanwhile, and their wait is limited).
 // (ms per SIMPLE iteration, grid / one CTA, by average rows per level: BFS 5k
 // 17: 188 / 117; cavity 40^2 20: 19 / 12; cavity 80^2 40: 84 / 70; hex 12^3 51:
 // 6.0 / 4.5; cavity 160^2 80: 172 / 211; hex 20^3 138: 9.7 / 14.6.)
-constexpr int SWEEP_WIDTH = 56;
+constexpr int SWEEP_WIDTH = 56, SWEEP_WIDEST = 16384;
 struct LevelLists {
   std::vector<int> frow, brow, items, ptr;
 };

@@ -78,6 +78,12 @@ struct MatT {
 };
 using Mat = MatT<double>;
 
+// Most levels that one CTA sweeps while the others wait at a barrier.  A wait
+// is limited (2 s unless the caller sets less), so the work inside one must not
+// grow with the mesh: 1024 levels of at most SWEEP_WIDEST rows (host_mesh.h),
+// about 1.2 ms for levels of a few dozen rows.  The barrier costs about 2 us.
+constexpr int SWEEP_WAIT = 1024;
+
 // CG in one cluster (xcal_cg_cluster_kernel): most threads of a CTA, vectors,
 // most tiles of the mesh (one partial per lane of the final sum) and of a CTA.
 // At 8 tiles a CTA makes two rounds of a phase; with more the resident form in
