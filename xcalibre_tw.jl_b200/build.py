@@ -30,6 +30,13 @@ UNITS = [("xcal_kernel.cu", tag, ["-DXCAL_INST=" + tag, f"-DXCAL_NS={ns}", f"-DX
 UNITS += [("xcal_kernel.cu", "s" + tag, ["-DXCAL_INST=" + tag, f"-DXCAL_NS={ns}", f"-DXCAL_T={t}",
                                          f"-DXCAL_MB={mb}", "-DXCAL_SERVE_ONLY"])
           for tag, (ns, t, mb) in INSTANCES.items() if mb == 4 and ns >= 2]
+# the same for numberings with sweeps by one CTA (2 CTAs/SM; the serving kernel 4)
+UNITS += [(src, pre + tag + "w", defs + ["-DXCAL_INST=" + tag + "w", "-DXCAL_ONE=true"])
+          for src, pre, tag, defs in
+          [("xcal_kernel.cu", "", tag, [f"-DXCAL_NS={ns}", f"-DXCAL_T={t}", f"-DXCAL_MB={mb}"])
+           for tag, (ns, t, mb) in INSTANCES.items() if mb == 2] +
+          [("xcal_kernel.cu", "s", tag, [f"-DXCAL_NS={ns}", f"-DXCAL_T={t}", f"-DXCAL_MB={mb}", "-DXCAL_SERVE_ONLY"])
+           for tag, (ns, t, mb) in INSTANCES.items() if mb == 4 and ns >= 2]]
 # the CG kernel of large meshes: Krylov value type, CTAs per SM
 UNITS += [("xcal_kernel.cu", tag, ["-DXCAL_INST=" + tag, "-DXCAL_T=" + t, "-DXCAL_MB=8", "-DXCAL_CG"])
           for tag, t in (("cd", "double"), ("cf", "float"))]

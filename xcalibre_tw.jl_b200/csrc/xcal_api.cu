@@ -975,7 +975,14 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   h.ring = h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU
                ? ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, c->occ, h.ntiles, c->nblocks)
                : 0;
-  if (h.sweep >= 0) h.sweep = sweep_bytes((size_t)h.n * c->ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), c->occ);
+  // the build for sweeps by one CTA has 2 CTAs per SM
+  int occ = c->occ, nblocks = c->nblocks;
+  if (h.sweep >= 0) {
+    h.sweep = sweep_bytes((size_t)h.n * c->ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 0);
+    if (occ && c->mode == SYNC_GRID) nblocks = std::min(nblocks, max_coresident_blocks(c->ns, 0, c->device));
+    if (occ && c->mode == SYNC_CLUSTER) nblocks = std::min(nblocks, max_cluster_blocks(c->ns, 0));
+    occ = 0;
+  }
   h.conv = c->conv;
   h.abort_nan = (c->flags & XCAL_FLAG_ABORT_ON_NAN) ? 1 : 0;
   barrier_knobs(h);
@@ -1010,7 +1017,7 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
                                    : launch_cg(mixed, cgb, &h, c->stream));
     }
   } else if (iters > 0) {
-    CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, -1, c->stream));
+    CUDA_TRY(c, launch_program(c->ns, mixed, occ, c->mode, nblocks, &h, prog, iters, -1, c->stream));
   }
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
   // results: one pinned block, one synchronisation
@@ -1767,7 +1774,10 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
   h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, gmres_ctas);   // the serving build: 4 CTAs per SM
-  if (h.sweep >= 0) h.sweep = sweep_bytes((size_t)h.n * c.ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 1);
+  if (h.sweep >= 0)   // the server's build has sweeps by one CTA unless it colours (xcal_serve_create)
+    h.sweep = renumber == XCAL_RENUMBER_COLOR
+                  ? -1
+                  : sweep_bytes((size_t)h.n * c.ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 1);
   h.phase = nullptr;
   h.bar = nullptr;   // the serving loop gives the case a barrier word when it starts
   out.prm = h;

@@ -8,6 +8,11 @@
 // A case runs on a group of CTAs numbered 0..vnb()-1 (vbid()): the whole grid
 // of an ordinary launch, or the CTAs the serving kernel (bottom of this file)
 // gives the case.
+//
+// XCAL_ONE: this unit is a build for numberings with sweeps by one CTA.
+#ifndef XCAL_ONE
+#define XCAL_ONE false
+#endif
 #include "xcal_device.cuh"
 #include "xcal_kernel.h"
 
@@ -136,6 +141,16 @@ __device__ __forceinline__ void ctx_mesh(Ctx &C, const KParams &P) {
   C.blev = P.blev;
 }
 
+// The mesh scalars and level arrays as the solvers read them: from the kernel's
+// parameters, each read a constant-bank operand that need not stay in a
+// register from one phase to the next; in the build whose solvers are called
+// out of line, from their copy.
+#if XCAL_ONE
+__device__ __forceinline__ const Ctx &mesh_of(const Ctx &C) { return C; }
+#else
+__device__ __forceinline__ const KParams &mesh_of(const Ctx &C) { return *C.P; }
+#endif
+
 template <typename T>
 __device__ __forceinline__ const MatT<T> &matU(const KParams &P) {
   if constexpr (sizeof(T) == 4) return P.AU32; else return P.AU;
@@ -166,7 +181,7 @@ __device__ __forceinline__ int own_tile(int m, int cnt, int rev) {
 
 template <class F>
 __device__ __forceinline__ void tile_each(const Ctx &C, F f) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const int cnt = own_tiles(P.ntiles);
   for (int m = 0; m < cnt; ++m) {
     const int i = own_tile(m, cnt, C.rev) * TILE + threadIdx.x;
@@ -182,7 +197,7 @@ __device__ __forceinline__ void tile_each(const Ctx &C, F f) {
 // warps are not held at a block barrier per tile.
 template <int K, class F>
 __device__ __forceinline__ void tile_phase(Ctx &C, bool reduce, F f) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const int nt = P.ntiles, cnt = own_tiles(nt), rev = C.rev;
   if (!reduce) {
     for (int m = 0; m < cnt; ++m) {
@@ -237,7 +252,8 @@ struct CgRows {
 // Row pairs pay when the CTAs hold two tiles or more each; with one tile per
 // CTA or fewer (small meshes: one phase is a barrier and one row per thread)
 // the one-row routines are faster.  Uniform across the CTAs of a run.
-__device__ __forceinline__ bool pairs_pay(const Ctx &P) { return P.ntiles >= 2 * vnb(); }
+template <class PT>
+__device__ __forceinline__ bool pairs_pay(const PT &P) { return P.ntiles >= 2 * vnb(); }
 
 // tile_phase over R tiles at a time: the CTA takes its tiles (in the phase's
 // direction) R by R, thread t row t of each (ii[r], ok[r] false past the
@@ -245,7 +261,7 @@ __device__ __forceinline__ bool pairs_pay(const Ctx &P) { return P.ntiles >= 2 *
 // those of tile_phase (each tile's canonical tree).
 template <int K, int R, class F>
 __device__ __forceinline__ void tile_phase_rows(Ctx &C, bool reduce, F f) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const int nt = P.ntiles, cnt = own_tiles(nt), rev = C.rev;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double *part = C.part_w();
@@ -527,8 +543,8 @@ __device__ __noinline__ void sweep_by_one(SweepArgs C, MatT<T> A, const T *in, T
 
 // Number of phases of M^{-1} after its producer phase.  The producer did the
 // row-local part (and, with first_lvl == 2, forward level 1 as well).
-template <typename T>
-__device__ __forceinline__ int precon_tail_phases(const Ctx &P, const MatT<T> &A, bool setup, int first_lvl) {
+template <class PT, typename T>
+__device__ __forceinline__ int precon_tail_phases(const PT &P, const MatT<T> &A, bool setup, int first_lvl) {
   if (!leveled(A)) return setup ? 1 : 0;
   return max(0, P.nfl - first_lvl) + (P.nbl - 1);
 }
@@ -539,7 +555,7 @@ __device__ __forceinline__ int precon_tail_phases(const Ctx &P, const MatT<T> &A
 // ONE: with the sweeps by one CTA for the numberings that have them.
 template <int NS, int K, bool ONE, typename T, class Red, int R = 1>
 __device__ __forceinline__ bool precon_tail(Ctx &C, const MatT<T> &A, const T *in, T *out, bool setup, int first_lvl, Red red) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const int nph = precon_tail_phases(P, A, setup, first_lvl);
   C.phase(setup ? PH_PREC_SETUP : PH_KRY_PREC);
   bool applied = nph == 0 && setup;   // nothing left to apply: reduce in a phase of its own
@@ -736,9 +752,11 @@ __device__ __forceinline__ bool krylov_start_inl(Ctx &C, const MatT<T> &A, const
   });
 }
 
-// A call inside the program costs its callers registers, so the numberings
-// with sweeps by one CTA have their own, out-of-line start, as they have the
-// out-of-line solvers.
+// A call inside the program costs all of it: a frame of 3 KB where 0.4 KB did,
+// and up to 0.4 us a phase (quad 157^2, p by BiCGSTAB: 1.80 -> 2.16 ms per
+// iteration).  So the numberings with sweeps by one CTA, whose time is in the
+// sweeps, have a build of the program of their own (ONE), with start and
+// solvers out of line; in the others everything is inlined.
 template <int NS, typename T>
 __device__ __noinline__ bool krylov_start_one(Ctx *state, MatT<T> A, KWorkT<T> w, const double *b, int solver) {
   Ctx C = *state;
@@ -746,9 +764,10 @@ __device__ __noinline__ bool krylov_start_one(Ctx *state, MatT<T> A, KWorkT<T> w
   *state = C;
   return ok;
 }
-template <int NS, typename T>
-__device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b, int solver) {
-  if (C.sweep < 0) return krylov_start_inl<NS, false, T>(C, A, w, b, solver);
+template <int NS, bool ONE, typename T>
+__device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
+                                             int solver) {
+  if constexpr (!ONE) return krylov_start_inl<NS, false, T>(C, A, w, b, solver);
   const KParams *P = C.P;
   Ctx t = C;
   t.P = nullptr;
@@ -771,7 +790,7 @@ __device__ __forceinline__ bool krylov_start(Ctx &C, const MatT<T> &A, const KWo
 template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool bicgstab(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *bb, const KCfg &cfg,
                          int (&its)[NS], double (&rnorm_out)[NS]) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   double red[2 * NS];
   final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
   double rho[NS], alpha[NS], omega[NS], beta[NS], rnorm[NS], eps[NS], nrho[NS];
@@ -1178,7 +1197,7 @@ __device__ __forceinline__ bool cg_two_level(Ctx &C, const MatT<T> &A, const KWo
 template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool cg(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                    double (&rnorm_out)[NS]) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const double EPS = 2.220446049250313e-16;
   double red[NS];
   final_sum<NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
@@ -1424,7 +1443,7 @@ __device__ __forceinline__ void sym_givens(double a, double b, double &c, double
 template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const KCfg &cfg, int (&its)[NS],
                       double (&rnorm_out)[NS]) {
-  const Ctx &P = C;
+  const auto &P = mesh_of(C);
   const double BTOL = 1.8189894035458565e-12;   // eps(Float64)^(3/4) = 2^-39
   double red[2 * NS];
   final_sum<2 * NS>(C.part_r(), P.ntiles, s_sm, s_out, red);
@@ -1601,7 +1620,7 @@ __device__ __forceinline__ bool gmres(Ctx &C, const MatT<T> &A, const KWorkT<T> 
   return true;
 }
 
-// The general solvers out of line, once per component count.  The state is
+// The solvers of the ONE build, once per component count.  The state is
 // copied in and back, so that the caller's own stays in registers; matrix and
 // vectors are read from shared memory (kept in registers they spilled).
 __shared__ __align__(16) unsigned char s_matrix[sizeof(Mat)], s_work[sizeof(KWork)];
@@ -1649,37 +1668,37 @@ __device__ __forceinline__ bool krylov(Ctx &C, const MatT<T> &A, const KWorkT<T>
   return ok;
 }
 
-// Solves of the program: the solvers inlined, where their operands are the
-// kernel's parameters (out of line a phase costs up to 0.7 us more); for the
-// numberings with sweeps by one CTA, whose time is in the sweeps, and for CG
-// on a vector out of line.
-template <int NS, typename T>
+template <int NS, bool ONE, typename T>
 __device__ __forceinline__ bool solve_vector(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
                                              const KCfg &cfg, int (&its)[NS], double (&rn)[NS]) {
-  if (cfg.solver == SOLVER_BICGSTAB && C.sweep < 0) return bicgstab<NS, false>(C, A, w, b, cfg, its, rn);
-  if (cfg.solver == SOLVER_GMRES && C.sweep < 0) return gmres<NS, false>(C, A, w, cfg, its, rn);
-  return krylov<NS, T>(C, A, w, b, cfg, its, rn);
+  if constexpr (ONE) {
+    return krylov<NS, T>(C, A, w, b, cfg, its, rn);
+  } else {
+    if (cfg.solver == SOLVER_BICGSTAB) return bicgstab<NS, false>(C, A, w, b, cfg, its, rn);
+    if (cfg.solver == SOLVER_GMRES) return gmres<NS, false>(C, A, w, cfg, its, rn);
+    return cg<NS, false>(C, A, w, cfg, its, rn);
+  }
 }
 
 // Pressure solve of a mesh of DIM dimensions.
-template <int DIM, typename T>
+template <int DIM, bool ONE, typename T>
 __device__ __forceinline__ bool solve_pressure(Ctx &C, const MatT<T> &A, const KWorkT<T> &w, const double *b,
                                                const KCfg &cfg, int (&its)[1], double (&rn)[1]) {
-  constexpr int WT = DIM == 2 ? 5 : DIM == 3 ? 7 : WUNROLL;   // rows of a quad or hex mesh
-  if (cfg.solver == SOLVER_CG && A.precon == PRECON_DILU && C.n0 > 0 && A.W <= WUNROLL) {
-    // (large meshes run the CG as a kernel of its own; here the rows of tiles
-    // that do not fit are those of a standalone solve or of a serving case)
-    if (C.ring * vnb() < C.ntiles) {
-#if defined(XCAL_SERVE_ONLY)
-      if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, false>(C, A, w, cfg, its[0], rn[0]);
-#endif
-      return cg_two_level<T, WUNROLL, false>(C, A, w, cfg, its[0], rn[0]);
+  if constexpr (!ONE) {   // a two-level numbering has no sweeps by one CTA
+    constexpr int WT = DIM == 2 ? 5 : DIM == 3 ? 7 : WUNROLL;   // rows of a quad or hex mesh
+    if (cfg.solver == SOLVER_CG && A.precon == PRECON_DILU && C.n0 > 0 && A.W <= WUNROLL) {
+      // (large meshes run the CG as a kernel of its own; here the rows of tiles
+      // that do not fit are those of a standalone solve, of a serving case or of
+      // a launch form that was asked for)
+      if (C.ring * vnb() < C.ntiles) {
+        if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, false>(C, A, w, cfg, its[0], rn[0]);
+        return cg_two_level<T, WUNROLL, false>(C, A, w, cfg, its[0], rn[0]);
+      }
+      if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, true>(C, A, w, cfg, its[0], rn[0]);
+      return cg_two_level<T, WUNROLL, true>(C, A, w, cfg, its[0], rn[0]);
     }
-    if (WT < WUNROLL && A.W == WT) return cg_two_level<T, WT, true>(C, A, w, cfg, its[0], rn[0]);
-    return cg_two_level<T, WUNROLL, true>(C, A, w, cfg, its[0], rn[0]);
   }
-  if (cfg.solver == SOLVER_CG && C.sweep < 0) return cg<1, false>(C, A, w, cfg, its, rn);
-  return solve_vector<1, T>(C, A, w, b, cfg, its, rn);
+  return solve_vector<1, ONE>(C, A, w, b, cfg, its, rn);
 }
 
 // -------------------------------------------------------------- assembly
@@ -2106,7 +2125,7 @@ __device__ __forceinline__ void bound_row(const KParams &P, double *fld, int i) 
   fld[i] = jmax(jmax(fi, average * (signbit(fi) ? 1.0 : 0.0)), EPS);
 }
 
-template <int NS, typename T>
+template <int NS, typename T, bool ONE>
 __device__ __forceinline__ bool turbulence(Ctx &C) {
   const KParams &P = *C.P;
   const double nu = P.nu;
@@ -2175,10 +2194,10 @@ __device__ __forceinline__ bool turbulence(Ctx &C) {
       krylov_init_row<1, T>(P, P.AP, A, wk, b, phi, i, cfg.solver);
     });
     if (!C.sync()) return false;
-    if (!krylov_start<1, T>(C, A, wk, P.bP, cfg.solver)) return false;
+    if (!krylov_start<1, ONE>(C, A, wk, P.bP, cfg.solver)) return false;
     int its[1];
     double rn[1];
-    if (!solve_vector<1, T>(C, A, wk, P.bP, cfg, its, rn)) return false;
+    if (!solve_vector<1, ONE>(C, A, wk, P.bP, cfg, its, rn)) return false;
     // run! copy-back, then constrain_boundary! for omega (:401-448)
     C.phase(PH_TURB);
     tile_each(C, [&](int i) {
@@ -2229,7 +2248,7 @@ __device__ __forceinline__ bool turbulence(Ctx &C) {
 // corr.  before_solve does everything between two solves up to the start of
 // solve k, after_solve everything that follows solve k-1 up to the end of its
 // corrector and, with the last corrector, of its iteration.
-template <int NS, typename T>
+template <int NS, typename T, bool ONE>
 struct Simple {
   Ctx &C;
   const bool piso;
@@ -2269,10 +2288,10 @@ struct Simple {
         krylov_init_row<NS, T>(P, P.AU, AUT, wU, b, P.U, i, P.kU.solver);
       });
       if (!C.sync()) return false;
-      if (!krylov_start<NS, T>(C, AUT, wU, P.bU, P.kU.solver)) return false;
+      if (!krylov_start<NS, ONE>(C, AUT, wU, P.bU, P.kU.solver)) return false;
       int itsU[NS];
       double rnU[NS];
-      if (!solve_vector<NS, T>(C, AUT, wU, P.bU, P.kU, itsU, rnU)) return false;
+      if (!solve_vector<NS, ONE>(C, AUT, wU, P.bU, P.kU, itsU, rnU)) return false;
 #pragma unroll
       for (int d = 0; d < NS; ++d) finite = finite && isfinite(rnU[d]);
       // run! copy-back: U = x + x0
@@ -2344,7 +2363,7 @@ struct Simple {
       krylov_init_row<1, T>(P, P.AP, APT, wP, b, P.p, i, P.kP.solver);
     });
     if (!C.sync()) return false;
-    return krylov_start<1, T>(C, APT, wP, P.bP, P.kP.solver);
+    return krylov_start<1, ONE>(C, APT, wP, P.bP, P.kP.solver);
   }
 
   // After solve k with `its` iterations and residual norm rn; stop: the run
@@ -2389,7 +2408,7 @@ struct Simple {
     grid_each(P.nf, [&](int f) { face_mdot<NS>(P, f); });
     if (!C.sync()) return false;
     if constexpr (NS == 2) {   // k-omega is a 2D model (xcal_case_setup refuses it in 3D)
-      if (P.model == 1 && !turbulence<NS, T>(C)) return false;
+      if (P.model == 1 && !turbulence<NS, T, ONE>(C)) return false;
     }
     if (corr + 1 < ncorr) return true;
     const bool lead = vbid() == 0 && threadIdx.x == 0;
@@ -2418,10 +2437,10 @@ struct Simple {
 // meshes, whose pressure solve is a kernel of its own (xcal_cg_kernel): launch
 // `step` does what follows solve step-1 and what leads to solve `step`, and
 // P.step carries the solve's results and the state of the run between them.
-template <int NS, typename T>
+template <int NS, typename T, bool ONE>
 __device__ __forceinline__ void simple_program(Ctx &C, int iters, bool piso, int step) {
   const KParams &P = *C.P;
-  Simple<NS, T> S{C, piso, piso ? 2 : 1, true};
+  Simple<NS, T, ONE> S{C, piso, piso ? 2 : 1, true};
   const int total = iters * S.ncorr;
   int its[1] = {0};
   double rn[1] = {0.0};
@@ -2447,10 +2466,11 @@ __device__ __forceinline__ void simple_program(Ctx &C, int iters, bool piso, int
       if (vbid() == 0 && threadIdx.x == 0) P.step->pw = C.pw;
       return;
     }
-    if (!solve_pressure<NS, T>(C, matP<T>(P), workP<T>(P), P.bP, P.kP, its, rn)) return;
+    if (!solve_pressure<NS, ONE>(C, matP<T>(P), workP<T>(P), P.bP, P.kP, its, rn)) return;
   }
 }
 
+template <bool ONE>
 __device__ __forceinline__ void solve_program(Ctx &C) {
   const KParams &P = *C.P;
   C.phase(PH_P_ASM);
@@ -2459,7 +2479,7 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
     krylov_init_row<1, double>(P, P.AU, P.AU, P.wU, b, P.U, i, P.solve_solver);
   });
   if (!C.sync()) return;
-  if (!krylov_start<1, double>(C, P.AU, P.wU, P.sb, P.solve_solver)) return;
+  if (!krylov_start<1, ONE>(C, P.AU, P.wU, P.sb, P.solve_solver)) return;
   KCfg cfg;
   cfg.solver = P.solve_solver;
   cfg.itmax = P.solve_itmax;
@@ -2467,7 +2487,7 @@ __device__ __forceinline__ void solve_program(Ctx &C) {
   cfg.rtol = P.solve_rtol;
   int its[1];
   double rn[1];
-  if (!solve_pressure<1, double>(C, P.AU, P.wU, P.sb, cfg, its, rn)) return;
+  if (!solve_pressure<1, ONE>(C, P.AU, P.wU, P.sb, cfg, its, rn)) return;
   tile_each(C, [&](int i) { P.U[i] = P.wU.x[i] + P.U[i]; });
   if (vbid() == 0 && threadIdx.x == 0) {
     P.solve_out[0] = (double)its[0];
@@ -2825,16 +2845,17 @@ __global__ void __launch_bounds__(CGC_TPB, 1) xcal_cg_cluster_kernel(const __gri
 // registers, few spills) suits meshes with about one tile per CTA, where a
 // phase is barrier-latency bound; 4 (64 registers, more spills, twice the
 // warps in flight) suits large meshes, where a phase is memory-latency bound.
-template <int NS, typename T, int MB>
+// ONE: the build for numberings with sweeps by one CTA (KParams::sweep >= 0).
+template <int NS, typename T, int MB, bool ONE>
 __global__ void __launch_bounds__(TPB, MB) xcal_program_kernel(const __grid_constant__ KParams prm, int prog, int iters,
                                                                int step) {
   if (step > 0 && (ld_volatile_i32(&prm.bar->err) || ld_volatile_i32(&prm.step->stop))) return;
   Ctx C;
   launch_begin(C, prm);
   if (prog == PROG_SOLVE) {
-    if constexpr (NS == 1 && sizeof(T) == 8) solve_program(C);
+    if constexpr (NS == 1 && sizeof(T) == 8) solve_program<ONE>(C);
   } else {
-    if constexpr (NS >= 2) simple_program<NS, T>(C, iters, prog == PROG_PISO, step);
+    if constexpr (NS >= 2) simple_program<NS, T, ONE>(C, iters, prog == PROG_PISO, step);
   }
   launch_end(C, prm, step >= 0);
 }
@@ -2863,7 +2884,7 @@ __device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned *p, unsigned v)
   return old;
 }
 
-template <int NS, typename T, int MB>
+template <int NS, typename T, int MB, bool ONE>
 __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, const ServeCtl *ctl) {
   __shared__ ServeJob sJ;   // the job record, read once per job
   __shared__ const ServeJob *s_job;
@@ -2948,7 +2969,7 @@ __global__ void __launch_bounds__(TPB, MB) xcal_serve_kernel(ServeMail *mail, co
     C.timers = false;
     C.tag = PH_SETUP;
     C.t_last = 0;
-    if (C.sync()) simple_program<NS, T>(C, J.iters, J.prog == PROG_PISO, -1);
+    if (C.sync()) simple_program<NS, T, ONE>(C, J.iters, J.prog == PROG_PISO, -1);
     C.sync();   // the run's results (fields, histories, done) complete
     // results to pinned host memory, this CTA's share
     {
@@ -3002,14 +3023,15 @@ const void *XCAL_CAT(cgc_kernel_, XCAL_INST)(int W) {
   return (const void *)xcal_cg_cluster_kernel<XCAL_T, WUNROLL>;
 }
 #elif defined(XCAL_SERVE_ONLY)
-template __global__ void xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB>(ServeMail *, const ServeCtl *);
+template __global__ void xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB, XCAL_ONE>(ServeMail *, const ServeCtl *);
 const void *XCAL_CAT(serve_kernel_, XCAL_INST)() {
-  return (const void *)xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB>;
+  return (const void *)xcal_serve_kernel<XCAL_NS, XCAL_T, XCAL_MB, XCAL_ONE>;
 }
 #else
-template __global__ void xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB>(const __grid_constant__ KParams, int, int, int);
+template __global__ void xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB, XCAL_ONE>(const __grid_constant__ KParams, int,
+                                                                                 int, int);
 const void *XCAL_CAT(program_kernel_, XCAL_INST)() {
-  return (const void *)xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB>;
+  return (const void *)xcal_program_kernel<XCAL_NS, XCAL_T, XCAL_MB, XCAL_ONE>;
 }
 #endif
 #endif

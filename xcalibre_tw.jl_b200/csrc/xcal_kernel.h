@@ -6,7 +6,8 @@
 
 namespace xcal {
 // occ selects the build: 0 = two resident CTAs per SM (128 registers),
-// 1 = four (64 registers); the NS = 1 standalone-solve program has only the first.
+// 1 = four (64 registers); the NS = 1 standalone-solve program and the builds for
+// sweeps by one CTA (taken where hparams->sweep >= 0) have only the first.
 cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, const KParams *hparams, int prog,
                            int iters, int step, cudaStream_t stream);
 // The pressure solve between two steps of a run (two-level numbering, row
@@ -32,6 +33,6 @@ const void *program_kernel_ptr(int ns, int mixed, int occ);
 void preload_programs();   // load every build on the current device
 // the serving kernel (xcal_serve_kernel) of a dimension and precision, and the
 // size of its launch on a device
-const void *serve_kernel_ptr(int ns, int mixed);
-int serve_grid(int ns, int mixed, int device);
+const void *serve_kernel_ptr(int ns, int mixed, int sweeps);
+int serve_grid(int ns, int mixed, int sweeps, int device);
 }  // namespace xcal

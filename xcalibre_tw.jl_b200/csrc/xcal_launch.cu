@@ -29,6 +29,16 @@ const void *serve_kernel_d2o();
 const void *serve_kernel_d3o();
 const void *serve_kernel_f2o();
 const void *serve_kernel_f3o();
+// builds for numberings with sweeps by one CTA
+const void *program_kernel_d1w();
+const void *program_kernel_d2w();
+const void *program_kernel_d3w();
+const void *program_kernel_f2w();
+const void *program_kernel_f3w();
+const void *serve_kernel_d2ow();
+const void *serve_kernel_d3ow();
+const void *serve_kernel_f2ow();
+const void *serve_kernel_f3ow();
 
 // Dynamic shared memory of the matrix tiles (cg_two_level) per CTA: what fits
 // beside the static part (5 KB) and the 1 KB the system keeps per CTA with 2
@@ -49,7 +59,9 @@ int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks) {
 int sweep_bytes(size_t bytes, int occ) { return (int)std::min(bytes, RING_BYTES[occ ? 1 : 0]); }
 
 // Serving kernel of a dimension and precision (4-CTA/SM builds).
-const void *serve_kernel_ptr(int ns, int mixed) {
+const void *serve_kernel_ptr(int ns, int mixed, int sweeps) {
+  if (sweeps && ns == 2) return mixed ? serve_kernel_f2ow() : serve_kernel_d2ow();
+  if (sweeps && ns == 3) return mixed ? serve_kernel_f3ow() : serve_kernel_d3ow();
   if (ns == 2) return mixed ? serve_kernel_f2o() : serve_kernel_d2o();
   if (ns == 3) return mixed ? serve_kernel_f3o() : serve_kernel_d3o();
   return nullptr;
@@ -77,8 +89,8 @@ size_t serve_dynamic_smem() { return RING_BYTES[1]; }
 
 // CTAs of the serving launch: every CTA that can be resident at once (a
 // cooperative launch of this size is guaranteed co-resident).
-int serve_grid(int ns, int mixed, int device) {
-  const void *fn = serve_kernel_ptr(ns, mixed);
+int serve_grid(int ns, int mixed, int sweeps, int device) {
+  const void *fn = serve_kernel_ptr(ns, mixed, sweeps);
   if (!fn) return 0;
   int per_sm = 0, sms = 0;
   if (allow_ring(fn, 1) != cudaSuccess ||
@@ -100,6 +112,13 @@ const void *program_kernel_ptr(int ns, int mixed, int occ) {
   return mixed ? program_kernel_f3() : program_kernel_d3();
 }
 
+// The program for a numbering with sweeps by one CTA: 2 CTAs per SM.
+static const void *sweep_kernel_ptr(int ns, int mixed) {
+  if (ns == 1) return program_kernel_d1w();
+  if (ns == 2) return mixed ? program_kernel_f2w() : program_kernel_d2w();
+  return mixed ? program_kernel_f3w() : program_kernel_d3w();
+}
+
 // Clusters above the portable 8 CTAs.
 static cudaError_t allow_large_clusters(const void *fn) {
   return allow_attribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -107,7 +126,7 @@ static cudaError_t allow_large_clusters(const void *fn) {
 
 cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, const KParams *hparams, int prog,
                            int iters, int step, cudaStream_t stream) {
-  const void *fn = program_kernel_ptr(ns, mixed, occ);
+  const void *fn = hparams->sweep >= 0 ? sweep_kernel_ptr(ns, mixed) : program_kernel_ptr(ns, mixed, occ);
   void *args[4];
   args[3] = (void *)&step;
   args[0] = (void *)hparams;

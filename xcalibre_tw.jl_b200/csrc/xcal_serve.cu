@@ -481,8 +481,9 @@ int xcal_serve_create(int device, const xcal_serve_cfg *cfg, xcal_server *out) {
   s->cfg = *cfg;
   if (cfg->tiles_per_cta > 0) s->tiles_per_cta = cfg->tiles_per_cta;
   if (cfg->max_ctas > 0) s->max_ctas = cfg->max_ctas;
-  s->kfn = xcal::serve_kernel_ptr(cfg->dim, cfg->precision == XCAL_PREC_MIXED);
-  s->grid = xcal::serve_grid(cfg->dim, cfg->precision == XCAL_PREC_MIXED, device);
+  const int sweeps = cfg->renumber != XCAL_RENUMBER_COLOR;   // coloured numberings have few and wide levels
+  s->kfn = xcal::serve_kernel_ptr(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps);
+  s->grid = xcal::serve_grid(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps, device);
   if (!s->kfn || s->grid < 1) {
     delete s;
     return XCAL_ERR_CUDA;
