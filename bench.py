@@ -6,9 +6,9 @@
 
 Default workload: the 3D lid-driven cavity, 128^3 hexahedra (2,097,152 cells),
 Re = 1000, steady SIMPLE with CG+DILU for p and BiCGSTAB+DILU for U (itmax 100,
-rtol 1e-3).  A step is one SIMPLE iteration (one launch of the persistent
-device program) continuing from the previous step, the run starting from zero
-fields as the case does.  K steps are timed in FP64 (`value`, the reference's
+rtol 1e-3).  A step is one SIMPLE iteration (the device program, cut in two
+launches where the pressure CG between them is a kernel of its own) continuing
+from the previous step, the run starting from zero fields as the case does.  K steps are timed in FP64 (`value`, the reference's
 arithmetic) and then, from the same initial fields, in mixed precision (FP32
 Krylov on FP64 assembly with FP64 residual refinement and dots); the line
 carries both rates, their ratio and the relative L2 difference of every field
@@ -45,17 +45,12 @@ sys.path.insert(0, os.path.join(ROOT, "xcalibre_tw.jl_b200"))
 METRIC = "SIMPLE cell-iters/s"
 UNIT = "cell-iters/s"
 RENUMBER = {"none": 0, "rcm": 1, "color": 2}
-
-
-def launches_per_step(cells, ns, renumber, precision):
-    """Kernels of one run(1): the program, or the program before and after the
-    pressure CG where that is a kernel of its own (two-colour numbering: small
-    meshes in one cluster, large ones beyond the program's shared memory)."""
-    tiles, width, size = -(-cells // 256), 7 if ns == 3 else 5, 4 if precision == "mixed" else 8
-    share = -(-tiles // 16)
-    cluster = share <= 8 and share * 256 * ((8 + width) * size + 4 * width) <= 220 * 1024
-    resident = tiles <= 148 * 4 * (48 * 1024 // (width * 256 * (size + 4)))
-    return 3 if renumber == "color" and (cluster or not resident) else 1
+# kernels of a step, by the form of its pressure solve
+CG_KERNEL = {"general": "xcal_program_kernel (SIMPLE iteration)",
+             "resident": "xcal_program_kernel (SIMPLE iteration)",
+             "streamed": "xcal_program_kernel (SIMPLE iteration)",
+             "cluster": "xcal_cg_cluster_kernel (pressure CG) between launches of xcal_program_kernel",
+             "kernel": "xcal_cg_kernel (pressure CG) between launches of xcal_program_kernel"}
 
 
 def parse():
@@ -123,11 +118,12 @@ def build_case(name, size=None, mesh_builder=None):
 
 
 # ------------------------------------------------------------ byte model
-def byte_model(mesh, kry, ns, sk=8):
+def byte_model(mesh, kry, ns, sk=8, two_level=False):
     """Algorithmic HBM bytes of one SIMPLE iteration per phase class
     (xcal._abi.PHASES) given its Krylov counts (kry: U iterations per
     component, p iterations at index 3); sk is the value size of the Krylov
-    iterations (8 FP64, 4 mixed).  Each phase class counts the minimum traffic
+    iterations (8 FP64, 4 mixed); two_level: the pressure CG over the two-colour
+    numbering, whose preconditioner phases touch half the rows each.  Each phase class counts the minimum traffic
     of its operations: every array it must read or write once.  Per-operation
     figures (s value size, k right-hand sides):
       SpMV (CSR)              nnz*(s+4) + (N+1)*4 + 2*k*N*s
@@ -166,9 +162,14 @@ def byte_model(mesh, kry, ns, sk=8):
     B["precon_setup"] = dilu_upd(sk) + dilu(ns, sk) + 2 * ns * N * sk + dilu_upd(sk) + dilu(1, sk) + 2 * N * sk
     # BiCGSTAB: phases A (p recomputed from r, p, v; q, p, M^-1 level 0 out) and D
     # (s from r, v; x += alpha p; q, s, t out); CG: phase A (p from z, p; p, q out)
-    B["krylov_spmv"] = (itU * (2 * spmv_mat(sk) + 14 * ns * N * sk) + itP * (spmv_mat(sk) + 4 * N * sk))
+    # (two levels: A reads z, p, x and writes p, q, x)
+    B["krylov_spmv"] = (itU * (2 * spmv_mat(sk) + 14 * ns * N * sk)
+                        + itP * (spmv_mat(sk) + (6 if two_level else 4) * N * sk))
     # BiCGSTAB: two M^-1 applications with their dots; CG: x/r update + M^-1 + <r,z>
-    B["krylov_precon"] = itU * (2 * dilu(ns, sk) + 4 * ns * N * sk) + itP * (dilu(1, sk) + 9 * N * sk)
+    # (two levels: B reads r, q, Dinv of all rows and writes r, z of level 1; C reads r, q, Dinv of level 0 and
+    # r, z of what it sums or gathers, and writes r, z of level 0)
+    B["krylov_precon"] = (itU * (2 * dilu(ns, sk) + 4 * ns * N * sk)
+                          + itP * (2 * Fi * (sk + 4) + 7 * N * sk if two_level else dilu(1, sk) + 9 * N * sk))
     B["krylov_vector"] = itU * 7 * ns * N * sk
     B["residual"] = spmv(ns, s) + 5 * ns * N * s + spmv(1, s) + N * s
     B["face"] = ((F * s * (1 + ns) + F * 16 + (1 + ns) * N * s)      # rDf, Uf(H)
@@ -541,8 +542,9 @@ def reference_main(a, rank):
 
 
 def run_timed(s, steps, dist, dev, flush, clk=None):
-    """K SIMPLE iterations, one launch each, event-timed on the library's
-    stream; returns per-step ms, Krylov counts and the phase timers' sums."""
+    """K SIMPLE iterations, one call each, event-timed on the library's stream;
+    returns per-step ms, Krylov counts, the phase timers' sums, and the form of
+    the pressure solve with the kernels launched."""
     import torch
     from xcal import _abi
     if dist:
@@ -550,6 +552,7 @@ def run_timed(s, steps, dist, dev, flush, clk=None):
     torch.cuda.synchronize(dev)
     ms, kry = [], []
     ph = {k: [0.0, 0] for k in _abi.PHASES}
+    form, launches = "general", 0
     for _ in range(steps):
         if flush is not None:
             flush.fill_(1.0)
@@ -557,23 +560,25 @@ def run_timed(s, steps, dist, dev, flush, clk=None):
         out = s.run(1)
         ms.append(s.last_ms())
         kry.append(out["krylov"][0])
+        f = s.last_form()
+        form, launches = f["cg"], launches + f["launches"]
         for k, (cyc, cnt) in s.last_phases().items():
             ph[k][0] += cyc
             ph[k][1] += cnt
     if dist:
         dist.barrier()
     torch.cuda.synchronize(dev)
-    return np.array(ms), np.array(kry), ph
+    return np.array(ms), np.array(kry), ph, form, launches
 
 
-def phase_table(mesh, ns, sk, ms, kry, ph, peak):
+def phase_table(mesh, ns, sk, ms, kry, ph, peak, two_level):
     """Per phase class: device time (the timers' cycle shares of the event-timed
     total), algorithmic bytes (byte_model with the measured Krylov counts) and
     the achieved fraction of the HBM peak."""
     from xcal import _abi
     bytes_ = {k: 0.0 for k in _abi.PHASES}
     for kr in kry:
-        for k, v in byte_model(mesh, kr, ns, sk).items():
+        for k, v in byte_model(mesh, kr, ns, sk, two_level).items():
             bytes_[k] += v
     total_cyc = sum(v[0] for v in ph.values())
     total_ms = float(ms.sum())
@@ -651,15 +656,16 @@ def main():
             s.run(1, want_krylov=False)
         reset(s)
         with ClockSampler(gpu_index) as clk:
-            ms, kry, ph = run_timed(s, a.steps, dist, dev, flush)
+            ms, kry, ph, form, launches = run_timed(s, a.steps, dist, dev, flush)
         if clocks is None:
             clocks = clk.summary()
         fields = {k: s.get_field(f) for k, f in (("Ux", _abi.FIELD_UX), ("Uy", _abi.FIELD_UY),
                                                   ("Uz", _abi.FIELD_UZ), ("p", _abi.FIELD_P))}
         total_ms = max_over_ranks(float(ms.sum()), dist, dev)
         sk = 4 if prec == _abi.PREC_MIXED else 8
-        table, total_bytes = phase_table(mesh, ns, sk, ms, kry, ph, peak)
-        runs[name] = dict(ms=ms, kry=kry, total_ms=total_ms, fields=fields, phases=table, tune=tune,
+        table, total_bytes = phase_table(mesh, ns, sk, ms, kry, ph, peak, form != "general")
+        runs[name] = dict(ms=ms, kry=kry, total_ms=total_ms, fields=fields, phases=table, tune=tune, form=form,
+                          launches=launches,
                           bytes_per_step=total_bytes / a.steps,
                           value=job_throughput(world, N * a.steps, total_ms / 1000.0))
         if solver_keep is None:
@@ -723,13 +729,13 @@ def main():
                    "parallelism": f"replicas x{world}"},
         "roofline": {"bound": "hbm", "achieved": frac, "peak": peak, "unit": "GB/s", "frac": frac / peak,
                      "peak_kind": peak_kind, "traffic": load_traffic(f"{a.config}_{N}_{main_name}_simple"),
-                     "kernel": "xcal_program_kernel (persistent SIMPLE iteration)"},
+                     "kernel": CG_KERNEL[R["form"]]},
         "phases": {k: v["phases"] for k, v in runs.items()},
         "autotune": {k: v["tune"] for k, v in runs.items()},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "steps": e2e_steps, "precision": main_name},
-        "gpu_launches": a.steps * launches_per_step(N, ns, a.renumber, main_name),
+        "gpu_launches": R["launches"],
         "clocks": clocks,
         "impl": "xcal",
     }

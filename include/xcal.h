@@ -220,7 +220,7 @@ int xcal_piso_run(xcal_ctx ctx, int32_t iterations, double *R_ux, double *R_uy,
  * class (components, power-of-two bucket of 256-cell tiles, matrix row width,
  * precision).  The case's fields are restored afterwards, so the tuning runs
  * leave no trace in the results.  Environment overrides (XCAL_SYNC, XCAL_OCC,
- * XCAL_NBLOCKS) take precedence over a remembered choice. */
+ * XCAL_NBLOCKS, XCAL_CG) take precedence over a remembered choice. */
 typedef struct {
   int32_t mode;             /* 1 hardware cluster barrier, 2 grid barrier */
   int32_t ctas;             /* CTAs of the launch */
@@ -257,6 +257,20 @@ enum {
 int xcal_last_run_stats(xcal_ctx ctx, double *ms, double *phase_cycles, int32_t nphases);
 /* Per-phase cycles and number of phases of each class in the last run. */
 int xcal_last_run_phases(xcal_ctx ctx, int32_t nphases, double *cycles, int64_t *count);
+
+/* What the last run launched: the form of its pressure solve (all forms compute
+ * the same values), its kernels (program and pressure solves), whether one CTA
+ * did its preconditioner sweeps, and the dynamic shared memory of a CTA of the
+ * program.  XCAL_CG=kernel, program or streamed in the environment asks for a
+ * form: a kernel of its own on the whole GPU (contexts with a grid barrier), one
+ * launch of the program, or that with the matrix rows left in global memory. */
+enum { XCAL_CG_GENERAL = 0,    /* the solver configured, in the program */
+       XCAL_CG_CLUSTER = 1,    /* CG over the two-colour numbering: one cluster, mesh in shared memory */
+       XCAL_CG_RESIDENT = 2,   /* in the program, matrix rows in shared memory */
+       XCAL_CG_STREAMED = 3,   /* in the program, matrix rows in global memory */
+       XCAL_CG_KERNEL = 4 };   /* a kernel on the whole GPU between launches of the program */
+typedef struct { int32_t cg, launches, sweeps_by_one, shared_bytes; } xcal_run_form;
+int xcal_last_run_form(xcal_ctx ctx, xcal_run_form *form);
 
 /* Assembled linear systems of the last iteration, in device numbering, CSR order:
  * which = 0 momentum (A shared by ux/uy/uz, b per component), 1 pressure.

@@ -71,6 +71,7 @@ struct xcal_ctx_s {
   double conv = 1e-7;          // SIMPLE stop tolerance
   int run_cap = 0;
   double last_ms = 0.0;
+  xcal_run_form form{};        // of the last run
   double *pin = nullptr;       // pinned staging, one region of n values per field
   size_t pin_n = 0;
   cudaEvent_t pin_ev[7] = {};  // last copy out of each pinned field region
@@ -238,7 +239,7 @@ static TuneKey tune_key(xcal_ctx c, int prec) {
 
 // A tuned form for this context's class, unless the environment forces one.
 static void apply_tuned(xcal_ctx c, int prec) {
-  if (getenv("XCAL_SYNC") || getenv("XCAL_OCC") || getenv("XCAL_NBLOCKS")) return;
+  if (getenv("XCAL_SYNC") || getenv("XCAL_OCC") || getenv("XCAL_NBLOCKS") || getenv("XCAL_CG")) return;
   if (c->flags & XCAL_FLAG_CLUSTER) return;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tune.find(tune_key(c, prec));
@@ -840,7 +841,7 @@ int xcal_case_setup(xcal_ctx c, const xcal_case *cfg) {
       !(c->flags & XCAL_FLAG_CLUSTER)) {
     const int mixed = h.prec == XCAL_PREC_MIXED;
     c->cgc = cg_cluster(mixed, h.AP.W, h.n0, h.ntiles);
-    if (c->cgc.ctas == 0) c->cg_ctas = cg_blocks(mixed, h.AP.W, c->device);
+    c->cg_ctas = cg_blocks(mixed, h.AP.W, c->device);
   }
   for (bool &b : c->pin_busy) b = false;
   c->d_stage = c->cbuf.alloc<double>((size_t)n * 7);
@@ -973,16 +974,18 @@ struct BatchState {
 // a limit of 1.)
 constexpr int BATCH_FIRST = 4, BATCH_MAX = 64;   // solves
 static int queue_cut_run(xcal_ctx c, const KParams &h, int prog, int iters, const CgCluster &cluster, int cg_ctas,
-                         BatchState *state) {
+                         BatchState *state, int32_t &launches) {
   const int mixed = h.prec == XCAL_PREC_MIXED;
   const int64_t total = (int64_t)iters * (prog == PROG_PISO ? 2 : 1);
   int64_t k = 0, size = BATCH_FIRST;
+  launches = 0;
   for (int batch = 0;; ++batch) {
     const int64_t end = std::min(total, k + size);
     for (; k < end; ++k) {
       CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, (int)k, c->stream));
       CUDA_TRY(c, cluster.ctas > 0 ? launch_cg_cluster(mixed, cluster, &h, c->stream)
                                    : launch_cg(mixed, cg_ctas, &h, c->stream));
+      launches += 2;
     }
     if (k == total) break;
     const int b = batch & 1;
@@ -995,6 +998,7 @@ static int queue_cut_run(xcal_ctx c, const KParams &h, int prog, int iters, cons
     size = std::min<int64_t>(BATCH_MAX, 2 * size);
   }
   CUDA_TRY(c, launch_program(c->ns, mixed, c->occ, c->mode, c->nblocks, &h, prog, iters, (int)total, c->stream));
+  launches += 1;
   return XCAL_OK;
 }
 
@@ -1020,7 +1024,8 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   h.mode = c->mode;
   // matrix rows in shared memory only for the solve that uses them: what it
   // takes is lost to L1 (cavity 64^3, BiCGSTAB for p: 3.7 -> 4.1 ms)
-  h.ring = h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU
+  const char *want = getenv("XCAL_CG");
+  h.ring = h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU && !(want && !strcmp(want, "streamed"))
                ? ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, c->occ, h.ntiles, c->nblocks)
                : 0;
   // the build for sweeps by one CTA has 2 CTAs per SM
@@ -1064,16 +1069,26 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   // Where the rows stop fitting, hexahedra FP64, ms per SIMPLE iteration: 66^3
   // in the program 2.48; 68^3 as a kernel 2.69, in the program 2.84.
   const int mixed = h.prec == XCAL_PREC_MIXED;
-  const bool own = iters > 0 && !getenv("XCAL_NBLOCKS") && !getenv("XCAL_SYNC");
+  const bool two_level = h.n0 > 0 && h.AP.W <= WUNROLL && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU;
+  const bool own = iters > 0 && !getenv("XCAL_NBLOCKS") && !getenv("XCAL_SYNC") && !want;
   const CgCluster cluster = own ? c->cgc : CgCluster{0, 0};
-  const int cgb = own && cluster.ctas == 0 && c->mode == SYNC_GRID && h.ring == 0 ? std::min(c->cg_ctas, h.ntiles) : 0;
+  const bool whole = (own && cluster.ctas == 0 && h.ring == 0) || (iters > 0 && want && !strcmp(want, "kernel"));
+  const int cgb = whole && c->mode == SYNC_GRID ? std::min(c->cg_ctas, h.ntiles) : 0;
+  c->form.cg = !two_level                        ? XCAL_CG_GENERAL
+               : cluster.ctas > 0                ? XCAL_CG_CLUSTER
+               : cgb > 0                         ? XCAL_CG_KERNEL
+               : h.ring * nblocks >= h.ntiles    ? XCAL_CG_RESIDENT
+                                                 : XCAL_CG_STREAMED;
+  c->form.sweeps_by_one = h.sweep >= 0;
+  c->form.launches = iters > 0;
   if (cluster.ctas > 0 || cgb > 0) {
     CUDA_TRY(c, cudaMemsetAsync(h.step, 0, sizeof(StepState), c->stream));
     h.ring = 0;   // the program's launches hold no matrix rows (a two-level numbering has no sweeps by one CTA)
-    TRY(queue_cut_run(c, h, prog, iters, cluster, cgb, batch));
+    TRY(queue_cut_run(c, h, prog, iters, cluster, cgb, batch, c->form.launches));
   } else if (iters > 0) {
     CUDA_TRY(c, launch_program(c->ns, mixed, occ, c->mode, nblocks, &h, prog, iters, -1, c->stream));
   }
+  c->form.shared_bytes = (int32_t)program_shared_bytes(mixed, h);
   CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
   Bar *hb = (Bar *)(batch + 2);
   int *hdn = (int *)(hb + 1);
@@ -1235,6 +1250,12 @@ int xcal_last_run_phases(xcal_ctx c, int32_t nph, double *cycles, int64_t *count
     if (cycles) cycles[i] = (i < NPH) ? (double)c->phase[i] : 0.0;
     if (count) count[i] = (i < NPH) ? (int64_t)c->phase[NPH + i] : 0;
   }
+  return XCAL_OK;
+}
+
+int xcal_last_run_form(xcal_ctx c, xcal_run_form *form) {
+  if (!c || !form) return XCAL_ERR_ARG;
+  *form = c->form;
   return XCAL_OK;
 }
 

@@ -24,6 +24,8 @@ cudaError_t launch_cg_cluster(int mixed, const CgCluster &form, const KParams *h
 // Matrix tiles of the launch's dynamic shared memory ring (KParams::ring).
 int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks);
 size_t serve_dynamic_smem();
+// Dynamic shared memory of a CTA of the program's launch.
+size_t program_shared_bytes(int mixed, const KParams &h);
 // Dynamic shared memory for the vector of a sweep by one CTA (a vector that
 // does not fit stays in global memory).
 int sweep_bytes(size_t bytes, int occ);

@@ -124,6 +124,11 @@ static cudaError_t allow_large_clusters(const void *fn) {
   return allow_attribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
+size_t program_shared_bytes(int mixed, const KParams &h) {
+  return std::max(h.ring * ring_tile_bytes(h.AU.W, mixed),   // one row width for both matrices
+                  (size_t)std::max(h.sweep, 0));
+}
+
 cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, const KParams *hparams, int prog,
                            int iters, int step, cudaStream_t stream) {
   const void *fn = hparams->sweep >= 0 ? sweep_kernel_ptr(ns, mixed) : program_kernel_ptr(ns, mixed, occ);
@@ -132,8 +137,7 @@ cudaError_t launch_program(int ns, int mixed, int occ, int mode, int nblocks, co
   args[0] = (void *)hparams;
   args[1] = (void *)&prog;
   args[2] = (void *)&iters;
-  const size_t dyn = std::max(hparams->ring * ring_tile_bytes(hparams->AU.W, mixed),   // one row width for both matrices
-                              (size_t)std::max(hparams->sweep, 0));
+  const size_t dyn = program_shared_bytes(mixed, *hparams);
   cudaError_t e = allow_ring(fn, occ);
   if (e != cudaSuccess) return e;
   if (mode == SYNC_BLOCK) return cudaLaunchKernel(fn, dim3(1), dim3(TPB), args, dyn, stream);

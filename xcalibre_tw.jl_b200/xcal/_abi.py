@@ -105,6 +105,13 @@ class TuneResult(C.Structure):
                 ("ms_default", C.c_double)]
 
 
+class RunForm(C.Structure):
+    _fields_ = [("cg", C.c_int32), ("launches", C.c_int32), ("sweeps_by_one", C.c_int32), ("shared_bytes", C.c_int32)]
+
+
+CG_FORMS = ("general", "cluster", "resident", "streamed", "kernel")
+
+
 class ServeCfg(C.Structure):
     _fields_ = [("slots", C.c_int32), ("max_iterations", C.c_int32), ("renumber", C.c_int32),
                 ("precision", C.c_int32), ("tolerance", C.c_double), ("dim", C.c_int32),
@@ -165,6 +172,7 @@ SIGNATURES = {
     "xcal_piso_run": (C.c_int, [C.c_void_p, C.c_int32, P_d, P_d, P_d, P_d, P_i32, P_i32]),
     "xcal_last_run_stats": (C.c_int, [C.c_void_p, P_d, P_d, C.c_int32]),
     "xcal_last_run_phases": (C.c_int, [C.c_void_p, C.c_int32, P_d, P_i64]),
+    "xcal_last_run_form": (C.c_int, [C.c_void_p, C.POINTER(RunForm)]),
     "xcal_autotune": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(TuneResult)]),
     "xcal_equation_get": (C.c_int, [C.c_void_p, C.c_int32, P_d, P_d, P_d, P_d]),
     "xcal_linear_solve": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int64, P_i32,

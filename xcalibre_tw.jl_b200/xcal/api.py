@@ -460,6 +460,15 @@ class Solver:
                    "xcal_last_run_phases")
         return {k: (float(cyc[i]), int(cnt[i])) for i, k in enumerate(_abi.PHASES)}
 
+    def last_form(self):
+        """What the last run launched: the form of its pressure solve
+        (_abi.CG_FORMS), its kernels, whether one CTA did its preconditioner
+        sweeps, and the program's dynamic shared memory per CTA."""
+        r = _abi.RunForm()
+        _abi.check(self.lib.xcal_last_run_form(self.ctx, C.byref(r)), self.ctx, "xcal_last_run_form")
+        return {"cg": _abi.CG_FORMS[r.cg], "launches": r.launches, "sweeps_by_one": bool(r.sweeps_by_one),
+                "shared_bytes": r.shared_bytes}
+
     def equation(self, which):
         n = self.n
         nnz = n + int(self.mesh.cell_faces_ptr[-1] - 1)
