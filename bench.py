@@ -8,15 +8,15 @@ Default workload: the 3D lid-driven cavity, 128^3 hexahedra (2,097,152 cells),
 Re = 1000, steady SIMPLE with CG+DILU for p and BiCGSTAB+DILU for U (itmax 100,
 rtol 1e-3).  A step is one SIMPLE iteration (the device program, cut in two
 launches where the pressure CG between them is a kernel of its own) continuing
-from the previous step, the run starting from zero fields as the case does.  K steps are timed in FP64 (`value`, the reference's
-arithmetic) and then, from the same initial fields, in mixed precision (FP32
-Krylov on FP64 assembly with FP64 residual refinement and dots); the line
-carries both rates, their ratio and the relative L2 difference of every field
-after the K steps.  The case's working set (about 2 GB) is far larger than the
-126 MB L2, so steps run back to back without an L2 flush; the smaller 2D
-workloads flush L2 (a 256 MiB write) between steps.  Each step is timed with
-CUDA events on the library's stream; per-phase device time comes from the
-library's phase timers (XCAL_FLAG_PHASE_TIMERS).
+from the previous step, the run starting from zero fields as the case does.  K
+steps are timed in FP64 (`value`, the reference's arithmetic) and then, from the
+same initial fields, in mixed precision (FP32 Krylov on FP64 assembly with FP64
+residual refinement and dots); the line carries both rates, their ratio and the
+relative L2 difference of every field after the K steps.  The case's working set
+(about 2 GB) is far larger than the 126 MB L2, so steps run back to back without
+an L2 flush; the smaller 2D workloads flush L2 (a 256 MiB write) between steps.
+Each step is timed with CUDA events on the library's stream; per-phase device
+time comes from the library's phase timers (XCAL_FLAG_PHASE_TIMERS).
 
 N > 1 runs N independent replicas (one per rank, weak scaling): a single case
 does not shard, and there is no collective on the data path.

@@ -544,9 +544,7 @@ static int mesh_arrays(xcal_ctx c, Sink &S) {
   h.f_sign = S.put_v(P.f_sign); h.f_first = S.put_v(P.f_first);
   h.cb_ptr = S.put_v(P.cb_ptr); h.cb_face = S.put_v(P.cb_face);
   h.flev = S.put_v(P.flev); h.blev = S.put_v(P.blev);
-  h.sweep = -1;
   if (!P.lists.frow.empty()) {
-    h.sweep = 0;
     h.frow = S.put_v(P.lists.frow); h.brow = S.put_v(P.lists.brow);
     h.items = S.put_v(P.lists.items); h.lptr = S.put_v(P.lists.ptr);
   }
@@ -955,6 +953,37 @@ int xcal_field_get(xcal_ctx c, int32_t field, double *host, int64_t n) {
   return XCAL_OK;
 }
 
+// KParams::sweep of the given solves (value bytes of the vector solved for,
+// preconditioner) on a mesh with lists for sweeps by one CTA: -1 where none of
+// them sweeps (the run then takes the build with everything inlined), else the dynamic
+// shared memory that the DILU sweeps of rows of at most WUNROLL entries use for
+// their vector: the largest that fits, and none for ILU(0), whose sweeps work in
+// global memory.  What is reserved is lost to L1 in every phase (quad 80^2 in the
+// caller's order, whose U does not fit: 49.8 ms per SIMPLE iteration with 96 KB
+// reserved all the same, 36.6 with what p takes; ILU(0) 64.4 / 44.6 with none).
+struct SweepUse {
+  size_t bytes;
+  int precon;
+};
+static int sweep_use(const KParams &h, int W, int occ, std::initializer_list<SweepUse> solves) {
+  if (!h.frow) return -1;
+  int use = -1;
+  for (const SweepUse &v : solves) {
+    if (v.precon != PRECON_DILU && v.precon != PRECON_ILU0) continue;
+    use = std::max(use, 0);
+    if (v.precon == PRECON_DILU && W <= WUNROLL && v.bytes == (size_t)sweep_bytes(v.bytes, occ))
+      use = std::max(use, (int)v.bytes);
+  }
+  return use;
+}
+// The solves of a case.
+static int sweep_use_case(const KParams &h, int ns, int occ) {
+  const size_t p = (size_t)h.n * (h.prec == XCAL_PREC_MIXED ? sizeof(float) : sizeof(double));
+  const bool turb = h.model == XCAL_MODEL_KOMEGA;
+  return sweep_use(h, h.AU.W, occ, {{p * ns, h.AU.precon}, {p, h.AP.precon}, {p, turb ? h.precK : h.AP.precon},
+                                    {p, turb ? h.precW : h.AP.precon}});
+}
+
 // -------------------------------------------------------------------- runs
 // State of a cut run after one of its batches, read back.
 struct BatchState {
@@ -1030,8 +1059,8 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
                : 0;
   // the build for sweeps by one CTA has 2 CTAs per SM
   int occ = c->occ, nblocks = c->nblocks;
+  h.sweep = sweep_use_case(h, c->ns, 0);
   if (h.sweep >= 0) {
-    h.sweep = sweep_bytes((size_t)h.n * c->ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 0);
     if (occ && c->mode == SYNC_GRID) nblocks = std::min(nblocks, max_coresident_blocks(c->ns, 0, c->device));
     if (occ && c->mode == SYNC_CLUSTER) nblocks = std::min(nblocks, max_cluster_blocks(c->ns, 0));
     occ = 0;
@@ -1066,8 +1095,11 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
   // launches of the program: in one cluster where the mesh fits its shared
   // memory, on the whole GPU where the matrix rows do not fit the CTAs' shared
   // memory.  (Launch forms asked for by the environment keep one launch.)
-  // Where the rows stop fitting, hexahedra FP64, ms per SIMPLE iteration: 66^3
-  // in the program 2.48; 68^3 as a kernel 2.69, in the program 2.84.
+  // Where the rows stop fitting the kernel takes over, whose warps hide the
+  // latency of HBM: 96^3 FP64 4.82 ms per SIMPLE iteration, 5.72 with streamed
+  // rows in the program; 101^3 mixed 4.73 / 5.47; 900^2 quads 4.98 / 5.45.  (While
+  // the solve still fits L2, up to about 70 MB, streamed rows in the program
+  // are faster: 66^3, resident, 2.06; 68^3 2.28 / 1.98; 76^3 2.99 / 2.92.)
   const int mixed = h.prec == XCAL_PREC_MIXED;
   const bool two_level = h.n0 > 0 && h.AP.W <= WUNROLL && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU;
   const bool own = iters > 0 && !getenv("XCAL_NBLOCKS") && !getenv("XCAL_SYNC") && !want;
@@ -1355,14 +1387,13 @@ int xcal_linear_solve(xcal_ctx c, int32_t solver, int32_t precon, int64_t n64, c
   h.nfl = nfl; h.nbl = nbl;
   h.n0 = two_level_rows(fl, n, nfl, nbl);
   const LevelLists lists = level_lists(fl, bl, n, nfl, nbl);
-  h.sweep = -1;
   if (!lists.frow.empty()) {
-    h.sweep = sweep_bytes((size_t)n * sizeof(double), 0);
     TRY(upload_c(c, B, h.frow, lists.frow)); TRY(upload_c(c, B, h.brow, lists.brow));
     TRY(upload_c(c, B, h.items, lists.items)); TRY(upload_c(c, B, h.lptr, lists.ptr));
   }
   TRY(upload_c(c, B, h.AU.col, ecol)); TRY(upload_c(c, B, h.AU.tpos, etp)); TRY(upload_c(c, B, h.AU.dpos, edp));
   h.AU.W = W; h.AU.np = np;
+  h.sweep = sweep_use(h, W, 0, {{(size_t)n * sizeof(double), precon}});
   std::vector<double> bb(b, b + n), xx(x, x + n);
   TRY(upload(c, B, h.AU.val, ev));
   TRY(upload(c, B, h.sb, bb));
@@ -1839,10 +1870,8 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
   h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, gmres_ctas);   // the serving build: 4 CTAs per SM
-  if (h.sweep >= 0)   // the server's build has sweeps by one CTA unless it colours (xcal_serve_create)
-    h.sweep = renumber == XCAL_RENUMBER_COLOR
-                  ? -1
-                  : sweep_bytes((size_t)h.n * c.ns * (h.prec == XCAL_PREC_MIXED ? 4 : 8), 1);
+  // the server's build has sweeps by one CTA unless it colours (xcal_serve_create)
+  h.sweep = renumber == XCAL_RENUMBER_COLOR ? -1 : sweep_use_case(h, c.ns, 1);
   h.phase = nullptr;
   h.bar = nullptr;   // the serving loop gives the case a barrier word when it starts
   out.prm = h;
