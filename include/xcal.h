@@ -216,9 +216,11 @@ int xcal_piso_run(xcal_ctx ctx, int32_t iterations, double *R_ux, double *R_uy,
 /* Autotuner (no reference counterpart): times `iterations` SIMPLE iterations
  * of the context's case in each launch form that computes the same values
  * (program build for 2 or 4 CTAs per SM, CTA count, hardware cluster or grid
- * barrier), keeps the fastest for the context, and remembers it for later contexts whose mesh falls in the same
- * class (components, power-of-two bucket of 256-cell tiles, matrix row width,
- * precision).  The case's fields are restored afterwards, so the tuning runs
+ * barrier), keeps the fastest for the context's case, and remembers it for later
+ * contexts whose mesh and case fall in the same class (components, power-of-two
+ * bucket of 256-cell tiles, matrix row width, precision, levels of the numbering,
+ * form of the pressure solve, model and solvers).  The case's fields are
+ * restored afterwards, so the tuning runs
  * leave no trace in the results.  Environment overrides (XCAL_SYNC, XCAL_OCC,
  * XCAL_NBLOCKS, XCAL_CG) take precedence over a remembered choice. */
 typedef struct {
@@ -260,7 +262,7 @@ int xcal_last_run_phases(xcal_ctx ctx, int32_t nphases, double *cycles, int64_t 
 
 /* What the last run launched: the form of its pressure solve (all forms compute
  * the same values), its kernels (program and pressure solves), whether one CTA
- * did its preconditioner sweeps, and the dynamic shared memory of a CTA of the
+ * did its preconditioner sweeps, and launch form and dynamic shared memory of the
  * program.  XCAL_CG=kernel, program or streamed in the environment asks for a
  * form: a kernel of its own on the whole GPU (contexts with a grid barrier), one
  * launch of the program, or that with the matrix rows left in global memory. */
@@ -269,7 +271,10 @@ enum { XCAL_CG_GENERAL = 0,    /* the solver configured, in the program */
        XCAL_CG_RESIDENT = 2,   /* in the program, matrix rows in shared memory */
        XCAL_CG_STREAMED = 3,   /* in the program, matrix rows in global memory */
        XCAL_CG_KERNEL = 4 };   /* a kernel on the whole GPU between launches of the program */
-typedef struct { int32_t cg, launches, sweeps_by_one, shared_bytes; } xcal_run_form;
+typedef struct {
+  int32_t cg, launches, sweeps_by_one, shared_bytes;
+  int32_t mode, ctas, ctas_per_sm;   /* of the program, as in xcal_tune_result */
+} xcal_run_form;
 int xcal_last_run_form(xcal_ctx ctx, xcal_run_form *form);
 
 /* Assembled linear systems of the last iteration, in device numbering, CSR order:

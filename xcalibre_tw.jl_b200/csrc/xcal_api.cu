@@ -50,6 +50,20 @@ struct DevBuf {
 
 }  // namespace
 
+// Class of a tuned launch form: components, tiles bucket = floor(log2 tiles),
+// row width, precision, and what decides which work the launch has: the levels
+// of the numbering, where the pressure is solved, and the solvers.
+struct TuneKey {
+  int ns, bucket, W, prec;
+  int levels;        // 0 two-level numbering, 1 sweeps by one CTA, 2 other
+  int form;          // pressure CG over two levels: 1 one cluster, 2 in the program, 3 its own kernel; 0 other
+  int64_t solvers;   // model, and solver and preconditioner of each equation
+  bool operator<(const TuneKey &o) const {
+    return std::tie(ns, bucket, W, prec, levels, form, solvers) <
+           std::tie(o.ns, o.bucket, o.W, o.prec, o.levels, o.form, o.solvers);
+  }
+};
+
 struct xcal_ctx_s {
   int device = 0;
   uint32_t flags = 0;
@@ -64,6 +78,8 @@ struct xcal_ctx_s {
   int ns = 2;
   int mode = SYNC_GRID, nblocks = 1;
   int occ = 0;                 // program build: 0 = 2 CTAs/SM, 1 = 4 CTAs/SM (xcal_kernel.h)
+  int mode0 = SYNC_GRID, occ0 = 0, nblocks0 = 1;   // the form chosen for the mesh, before any tuning
+  TuneKey tkey{};              // class of the case
   CgCluster cgc{0, 0};         // pressure CG in one cluster: its form for the case (0 CTAs: not)
   int cg_ctas = 0;             // pressure CG as a kernel on the whole GPU: its CTAs
   DevBuf mbuf, cbuf, rbuf;     // mesh, case, run buffers
@@ -213,36 +229,46 @@ static void barrier_knobs(KParams &h) {
 
 static void choose_launch_mode(xcal_ctx c, int n);
 
-// Launch forms chosen by xcal_autotune, per mesh class: (components, tiles
-// bucket = floor(log2 tiles), row width, precision).  A context whose mesh
-// falls in a tuned class starts with the tuned form (the environment
-// overrides of choose_launch_mode still win).  All forms compute the same
-// values; only the time differs.
-struct TuneKey {
-  int ns, bucket, W, prec;
-  bool operator<(const TuneKey &o) const {
-    return std::tie(ns, bucket, W, prec) < std::tie(o.ns, o.bucket, o.W, o.prec);
-  }
-};
+// Launch forms chosen by xcal_autotune, per class (TuneKey).  A context whose
+// mesh and case fall in a tuned class starts with the tuned form (the
+// environment overrides of choose_launch_mode still win).  All forms compute
+// the same values; only the time differs.
 struct TuneChoice {
   int mode, occ, nblocks;
 };
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneChoice> g_tune;
 
-static TuneKey tune_key(xcal_ctx c, int prec) {
+static TuneKey tune_key(xcal_ctx c, const xcal_case &cfg) {
   const int ntiles = (c->prep.n + TILE - 1) / TILE;
   int b = 0;
   while ((2 << b) <= ntiles) ++b;
-  return TuneKey{c->ns, b, c->prep.W, prec};
+  const Prep &P = c->prep;
+  const int mixed = cfg.precision == XCAL_PREC_MIXED;
+  int form = 0;
+  if (P.n0 > 0 && P.W <= WUNROLL && cfg.solver_p.solver == XCAL_SOLVER_CG &&
+      cfg.solver_p.preconditioner == XCAL_PRECON_DILU) {
+    if (cg_cluster(mixed, P.W, P.n0, ntiles).ctas > 0) form = 1;
+    else form = ring_tiles(P.W, mixed, c->occ0, ntiles, c->nblocks0) > 0 ? 2 : 3;
+  }
+  int64_t solvers = cfg.model;
+  const xcal_solver_cfg *eq[4] = {&cfg.solver_U, &cfg.solver_p, &cfg.solver_k, &cfg.solver_omega};
+  for (int q = 0; q < (cfg.model == XCAL_MODEL_KOMEGA ? 4 : 2); ++q)
+    solvers = solvers * 64 + eq[q]->solver * 8 + eq[q]->preconditioner;
+  return TuneKey{c->ns, b, P.W, cfg.precision, P.n0 > 0 ? 0 : P.lists.frow.empty() ? 2 : 1, form, solvers};
 }
 
 // A tuned form for this context's class, unless the environment forces one.
-static void apply_tuned(xcal_ctx c, int prec) {
+// (A form tuned for a case that the context held before is given up.)
+static void apply_tuned(xcal_ctx c, const xcal_case &cfg) {
+  c->tkey = tune_key(c, cfg);
   if (getenv("XCAL_SYNC") || getenv("XCAL_OCC") || getenv("XCAL_NBLOCKS") || getenv("XCAL_CG")) return;
   if (c->flags & XCAL_FLAG_CLUSTER) return;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  auto it = g_tune.find(tune_key(c, prec));
+  c->mode = c->mode0;
+  c->occ = c->occ0;
+  c->nblocks = c->nblocks0;
+  auto it = g_tune.find(c->tkey);
   if (it == g_tune.end()) return;
   c->mode = it->second.mode;
   c->occ = it->second.occ;
@@ -570,6 +596,9 @@ int xcal_mesh_upload(xcal_ctx c, const xcal_mesh_desc *d, int32_t renumber) {
   DevSink S(c, c->mbuf);
   TRY(mesh_arrays(c, S));
   choose_launch_mode(c, c->prep.n);
+  c->mode0 = c->mode;
+  c->occ0 = c->occ;
+  c->nblocks0 = c->nblocks;
   {
     std::vector<int> p32(c->perm.begin(), c->perm.end());
     c->d_perm = S.put_v(p32);
@@ -821,7 +850,7 @@ int xcal_case_setup(xcal_ctx c, const xcal_case *cfg) {
   c->run_cap = 0;
   KParams &h = c->hp;
   int n = c->prep.n;
-  apply_tuned(c, cfg->precision);
+  apply_tuned(c, *cfg);
   DevSink B(c, c->cbuf);
   TRY(case_arrays(c, cfg, B, nullptr, nullptr));
   h.bar = B.scratch_n<Bar>(1);
@@ -1113,6 +1142,9 @@ static int run_program(xcal_ctx c, int prog, int32_t iters, double *Rux, double 
                                                  : XCAL_CG_STREAMED;
   c->form.sweeps_by_one = h.sweep >= 0;
   c->form.launches = iters > 0;
+  c->form.mode = c->mode;
+  c->form.ctas = nblocks;
+  c->form.ctas_per_sm = occ ? 4 : 2;
   if (cluster.ctas > 0 || cgb > 0) {
     CUDA_TRY(c, cudaMemsetAsync(h.step, 0, sizeof(StepState), c->stream));
     h.ring = 0;   // the program's launches hold no matrix rows (a two-level numbering has no sweeps by one CTA)
@@ -1257,7 +1289,7 @@ int xcal_autotune(xcal_ctx c, int32_t iters, xcal_tune_result *out) {
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[tune_key(c, h.prec)] = TuneChoice{b.mode, b.occ, b.nblocks};
+    g_tune[c->tkey] = TuneChoice{b.mode, b.occ, b.nblocks};
   }
   out->mode = b.mode;
   out->ctas = b.nblocks;

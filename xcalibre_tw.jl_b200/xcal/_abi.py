@@ -106,7 +106,8 @@ class TuneResult(C.Structure):
 
 
 class RunForm(C.Structure):
-    _fields_ = [("cg", C.c_int32), ("launches", C.c_int32), ("sweeps_by_one", C.c_int32), ("shared_bytes", C.c_int32)]
+    _fields_ = [("cg", C.c_int32), ("launches", C.c_int32), ("sweeps_by_one", C.c_int32), ("shared_bytes", C.c_int32),
+                ("mode", C.c_int32), ("ctas", C.c_int32), ("ctas_per_sm", C.c_int32)]
 
 
 CG_FORMS = ("general", "cluster", "resident", "streamed", "kernel")

@@ -463,11 +463,12 @@ class Solver:
     def last_form(self):
         """What the last run launched: the form of its pressure solve
         (_abi.CG_FORMS), its kernels, whether one CTA did its preconditioner
-        sweeps, and the program's dynamic shared memory per CTA."""
+        sweeps, and the program's launch form and dynamic shared memory per CTA."""
         r = _abi.RunForm()
         _abi.check(self.lib.xcal_last_run_form(self.ctx, C.byref(r)), self.ctx, "xcal_last_run_form")
-        return {"cg": _abi.CG_FORMS[r.cg], "launches": r.launches, "sweeps_by_one": bool(r.sweeps_by_one),
-                "shared_bytes": r.shared_bytes}
+        out = {k: getattr(r, k) for k, _ in _abi.RunForm._fields_}
+        out["cg"], out["sweeps_by_one"] = _abi.CG_FORMS[r.cg], bool(r.sweeps_by_one)
+        return out
 
     def equation(self, which):
         n = self.n
