@@ -433,6 +433,7 @@ typedef struct {
   double device_bytes;      /* device arena size */
   double device_bytes_peak; /* most arena memory held by admitted cases at once */
   int64_t grid_ctas;        /* CTAs of the serving launch */
+  int64_t resident;         /* cases set up to keep the matrix rows of the pressure CG in shared memory */
 } xcal_serve_stats;
 int xcal_serve_create(int device, const xcal_serve_cfg *cfg, xcal_server *out);
 /* U0 holds ux, uy, uz (3 x ncells, the caller's cell order); p0 ncells.

@@ -1869,9 +1869,9 @@ int xcal_viscous_force(xcal_ctx c, int32_t patch, double rho, double F[3]) {
 namespace xcal {
 
 int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *cfg, const double *U0,
-                     const double *p0, double tolerance, int iters, int gmres_ctas, Sink &sink, CaseImage &out,
-                     std::string &err) {
-  if (!mesh || !cfg || !U0 || !p0 || iters < 1 || gmres_ctas < 1) {
+                     const double *p0, double tolerance, int iters, const ServeGroup &group, Sink &sink,
+                     CaseImage &out, std::string &err) {
+  if (!mesh || !cfg || !U0 || !p0 || iters < 1 || group.tiles_per_cta < 1 || group.max_ctas < 1) {
     err = "bad case image arguments";
     return XCAL_ERR_ARG;
   }
@@ -1881,7 +1881,8 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   if (st == XCAL_OK) st = check_case(&c, cfg);
   if (st == XCAL_OK) {
     c.mode = SYNC_GRID;
-    c.nblocks = gmres_ctas;   // GMRES per-CTA scratch
+    const int tiles = c.hp.ntiles;
+    c.nblocks = std::max(1, std::min((tiles + group.tiles_per_cta - 1) / group.tiles_per_cta, group.max_ctas));
     st = mesh_arrays(&c, sink);
   }
   if (st == XCAL_OK) st = case_arrays(&c, cfg, sink, U0, p0);
@@ -1901,7 +1902,10 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.conv = tolerance;
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
-  h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, gmres_ctas);   // the serving build: 4 CTAs per SM
+  // rows of the case's own group: 40 tiles on 10 CTAs hold 4 each
+  if (h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU)
+    h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, c.nblocks);
+  if (program_shared_bytes(h.prec == XCAL_PREC_MIXED, h) > group.shared_bytes) h.ring = 0;
   // the server's build has sweeps by one CTA unless it colours (xcal_serve_create)
   h.sweep = renumber == XCAL_RENUMBER_COLOR ? -1 : sweep_use_case(h, c.ns, 1);
   h.phase = nullptr;
@@ -1909,7 +1913,8 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   out.prm = h;
   out.ns = c.ns;
   out.n = c.prep.n;
-  out.ntiles = h.ntiles;
+  out.ctas = c.nblocks;
+  out.resident = h.ring > 0;
   out.perm = c.perm;
   return XCAL_OK;
 }

@@ -86,18 +86,26 @@ struct CaseImage {
   KParams prm;
   int ns = 2;
   int64_t n = 0;              // cells
-  int ntiles = 0;
+  int ctas = 0;               // CTAs of its group
+  bool resident = false;      // the pressure CG keeps its matrix rows in shared memory
   std::vector<int64_t> perm;  // caller cell -> device cell
   std::vector<double> uz;     // z velocity of a 2D case (unchanged by the run)
+};
+
+// How a server groups its CTAs: the tiles a CTA is given, the largest group, and
+// the dynamic shared memory of a CTA.
+struct ServeGroup {
+  int tiles_per_cta, max_ctas;
+  size_t shared_bytes;
 };
 
 // Builds `cfg` on the mesh `mesh` (host descriptor) into `sink`, with the
 // initial fields U0 (3 x n, caller order) and p0: renumbering, layout, BC
 // tables, work arrays, run arrays for `iters` iterations.  Runs twice per
 // case: a measure pass, then the build pass into the allocated region.
-// gmres_ctas: CTAs the GMRES scratch is sized for.
+// The image is for the group that the case gets: out.ctas.
 int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *cfg, const double *U0,
-                     const double *p0, double tolerance, int iters, int gmres_ctas, Sink &sink, CaseImage &out,
-                     std::string &err);
+                     const double *p0, double tolerance, int iters, const ServeGroup &group, Sink &sink,
+                     CaseImage &out, std::string &err);
 
 }  // namespace xcal

@@ -23,7 +23,6 @@ CgCluster cg_cluster(int mixed, int W, int n0, int ntiles);
 cudaError_t launch_cg_cluster(int mixed, const CgCluster &form, const KParams *hparams, cudaStream_t stream);
 // Matrix tiles of the launch's dynamic shared memory ring (KParams::ring).
 int ring_tiles(int W, int mixed, int occ, int ntiles, int nblocks);
-size_t serve_dynamic_smem();
 // Dynamic shared memory of a CTA of the program's launch.
 size_t program_shared_bytes(int mixed, const KParams &h);
 // Dynamic shared memory for the vector of a sweep by one CTA (a vector that
@@ -34,7 +33,8 @@ int max_cluster_blocks(int ns, int occ = 0);
 const void *program_kernel_ptr(int ns, int mixed, int occ);
 void preload_programs();   // load every build on the current device
 // the serving kernel (xcal_serve_kernel) of a dimension and precision, and the
-// size of its launch on a device
+// dynamic shared memory and size of its launch on a device
 const void *serve_kernel_ptr(int ns, int mixed, int sweeps);
-int serve_grid(int ns, int mixed, int sweeps, int device);
+size_t serve_shared_bytes(int ns, int mixed, int sweeps, int tiles_per_cta);
+int serve_grid(int ns, int mixed, int sweeps, size_t shared_bytes, int device);
 }  // namespace xcal

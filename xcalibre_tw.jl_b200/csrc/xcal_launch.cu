@@ -85,16 +85,26 @@ static cudaError_t allow_ring(const void *fn, int occ) {
   return allow_attribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RING_BYTES[occ ? 1 : 0]);
 }
 
-size_t serve_dynamic_smem() { return RING_BYTES[1]; }
+// Dynamic shared memory of a CTA of the serving launch: the matrix rows of a
+// full CTA (quads, hexahedra) where they fit, else none, which leaves the L1 to
+// rows read from global memory; the vector of the sweeps by one CTA.
+// (16 cases of up to 160 tiles, 300 iterations, mean run of a case: mixed 696 ms
+// streamed beside 48 KB, 625 resident; FP64, whose 4 tiles do not fit, 730
+// beside 48 KB reserved for nothing, 650 with none.)
+size_t serve_shared_bytes(int ns, int mixed, int sweeps, int tiles_per_cta) {
+  if (sweeps) return RING_BYTES[1];
+  const size_t rows = (size_t)tiles_per_cta * ring_tile_bytes(ns == 3 ? 7 : 5, mixed);
+  return rows <= RING_BYTES[1] ? rows : 0;
+}
 
 // CTAs of the serving launch: every CTA that can be resident at once (a
 // cooperative launch of this size is guaranteed co-resident).
-int serve_grid(int ns, int mixed, int sweeps, int device) {
+int serve_grid(int ns, int mixed, int sweeps, size_t shared_bytes, int device) {
   const void *fn = serve_kernel_ptr(ns, mixed, sweeps);
   if (!fn) return 0;
   int per_sm = 0, sms = 0;
   if (allow_ring(fn, 1) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, serve_dynamic_smem()) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, shared_bytes) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;

@@ -129,7 +129,7 @@ struct Job {
 struct xcal_server_s {
   int device = 0;
   xcal_serve_cfg cfg{};
-  int tiles_per_cta = 4, max_ctas = 64;
+  xcal::ServeGroup group{4, 64, 0};
   // device arena, pinned host arena (with its device view), barrier words
   char *dev_arena = nullptr;
   char *host_arena = nullptr, *host_arena_dev = nullptr;
@@ -164,11 +164,6 @@ struct xcal_server_s {
 
 namespace {
 
-int choose_k(xcal_server s, int ntiles) {
-  int k = (ntiles + s->tiles_per_cta - 1) / s->tiles_per_cta;
-  return std::max(1, std::min(std::min(k, s->max_ctas), s->grid));
-}
-
 // Image of one case: measure pass, admission (device and host footprint),
 // build pass into the allocated regions, job record.
 int setup_job(xcal_server s, Job &j) {
@@ -182,7 +177,7 @@ int setup_job(xcal_server s, Job &j) {
   ImageSink meas;
   CaseImage tmp;
   st = xcal::build_case_image(&d, s->cfg.renumber, &cfg, j.U0.data(), j.p0.data(), s->cfg.tolerance, iters,
-                              s->max_ctas, meas, tmp, e);
+                              s->group, meas, tmp, e);
   if (st) return st;
   if (tmp.ns != s->cfg.dim) return XCAL_ERR_UNSUPPORTED;
   if (cfg.model != XCAL_MODEL_LAMINAR) return XCAL_ERR_UNSUPPORTED;
@@ -215,7 +210,7 @@ int setup_job(xcal_server s, Job &j) {
   b.dev_base = s->dev_arena + j.dev_off;
   b.host_img = s->host_arena + j.host_off;
   st = xcal::build_case_image(&d, s->cfg.renumber, &cfg, j.U0.data(), j.p0.data(), s->cfg.tolerance, iters,
-                              s->max_ctas, b, j.img, e);
+                              s->group, b, j.img, e);
   if (st || b.copy_off > b.copy_size || b.zero_off > b.zero_size || b.scratch_off > b.scratch_size) {
     std::lock_guard<std::mutex> lk(s->mu);
     s->dalloc.release(j.dev_off, j.dev_bytes);
@@ -252,7 +247,7 @@ int setup_job(xcal_server s, Job &j) {
   J.out_R = (double *)dev_of(j.oR);
   J.out_kry = (int *)dev_of(j.okry);
   J.out_state = (int *)dev_of(j.state);
-  j.k = choose_k(s, j.img.ntiles);
+  j.k = j.img.ctas;
   return XCAL_OK;
 }
 
@@ -301,6 +296,7 @@ void setup_main(xcal_server s) {
       s->cv_done.notify_all();
       continue;
     }
+    s->st.resident += j->img.resident;
     s->ready.push_back(j);
     s->cv_sched.notify_all();
   }
@@ -441,7 +437,8 @@ void sched_main(xcal_server s) {
 
 int launch_server_kernel(xcal_server s) {
   void *args[2] = {(void *)&s->mail_dev, (void *)&s->ctl_dev};
-  cudaError_t e = cudaLaunchCooperativeKernel(s->kfn, dim3(s->grid), dim3(xcal::TPB), args, xcal::serve_dynamic_smem(), s->kstream);
+  cudaError_t e = cudaLaunchCooperativeKernel(s->kfn, dim3(s->grid), dim3(xcal::TPB), args,
+                                              s->group.shared_bytes, s->kstream);
   if (e != cudaSuccess) return XCAL_ERR_CUDA;
   if (cudaEventRecord(s->kdone, s->kstream) != cudaSuccess) return XCAL_ERR_CUDA;
   s->kernel_live = true;
@@ -479,16 +476,18 @@ int xcal_serve_create(int device, const xcal_serve_cfg *cfg, xcal_server *out) {
   auto *s = new xcal_server_s();
   s->device = device;
   s->cfg = *cfg;
-  if (cfg->tiles_per_cta > 0) s->tiles_per_cta = cfg->tiles_per_cta;
-  if (cfg->max_ctas > 0) s->max_ctas = cfg->max_ctas;
+  if (cfg->tiles_per_cta > 0) s->group.tiles_per_cta = cfg->tiles_per_cta;
+  if (cfg->max_ctas > 0) s->group.max_ctas = cfg->max_ctas;
   const int sweeps = cfg->renumber != XCAL_RENUMBER_COLOR;   // coloured numberings have few and wide levels
   s->kfn = xcal::serve_kernel_ptr(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps);
-  s->grid = xcal::serve_grid(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps, device);
+  s->group.shared_bytes =
+      xcal::serve_shared_bytes(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps, s->group.tiles_per_cta);
+  s->grid = xcal::serve_grid(cfg->dim, cfg->precision == XCAL_PREC_MIXED, sweeps, s->group.shared_bytes, device);
   if (!s->kfn || s->grid < 1) {
     delete s;
     return XCAL_ERR_CUDA;
   }
-  s->max_ctas = std::min(s->max_ctas, s->grid);
+  s->group.max_ctas = std::min(s->group.max_ctas, s->grid);
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) {
     delete s;

@@ -130,7 +130,7 @@ class ServeStats(C.Structure):
     _fields_ = [("submitted", C.c_int64), ("completed", C.c_int64), ("failed", C.c_int64),
                 ("queued", C.c_int64), ("running", C.c_int64), ("cell_iterations", C.c_double),
                 ("run_ms", C.c_double), ("device_bytes", C.c_double), ("device_bytes_peak", C.c_double),
-                ("grid_ctas", C.c_int64)]
+                ("grid_ctas", C.c_int64), ("resident", C.c_int64)]
 
 
 def dptr(a):
