@@ -202,7 +202,8 @@ int xcal_field_set(xcal_ctx ctx, int32_t field, const double *host, int64_t n);
 int xcal_field_get(xcal_ctx ctx, int32_t field, double *host, int64_t n);
 
 /* simple!(model, config; pref) -> (R_ux, R_uy, R_p): src/Solvers/Solvers_1_SIMPLE.jl:3-231.
- * Runs `iterations` SIMPLE iterations (one persistent device kernel), writes the
+ * Runs `iterations` SIMPLE iterations (one persistent device kernel, or launches of
+ * it with the pressure solves between them: xcal_last_run_form), writes the
  * residual histories (entries after convergence stay 1.0 as in the reference),
  * and optionally the Krylov iteration count of every solve (krylov_iters has
  * 5*iterations entries: ux, uy, uz, p, spare; may be NULL).  *done receives the
@@ -433,7 +434,6 @@ typedef struct {
   double device_bytes;      /* device arena size */
   double device_bytes_peak; /* most arena memory held by admitted cases at once */
   int64_t grid_ctas;        /* CTAs of the serving launch */
-  int64_t resident;         /* cases set up to keep the matrix rows of the pressure CG in shared memory */
 } xcal_serve_stats;
 int xcal_serve_create(int device, const xcal_serve_cfg *cfg, xcal_server *out);
 /* U0 holds ux, uy, uz (3 x ncells, the caller's cell order); p0 ncells.
@@ -449,6 +449,8 @@ int xcal_serve_submit(xcal_server s, const xcal_mesh_desc *mesh, const xcal_case
 int xcal_serve_poll(xcal_server s, int64_t ticket, int32_t wait_ms, xcal_serve_result *res,
                     double *U, double *p);
 int xcal_serve_stats_get(xcal_server s, xcal_serve_stats *st);
+/* Cases set up so far that keep the matrix rows of the pressure CG in shared memory. */
+int xcal_serve_resident(xcal_server s, int64_t *cases);
 /* Finishes the running cases, drops the queued ones, ends the launch. */
 int xcal_serve_destroy(xcal_server s);
 

@@ -248,7 +248,7 @@ static TuneKey tune_key(xcal_ctx c, const xcal_case &cfg) {
   int form = 0;
   if (P.n0 > 0 && P.W <= WUNROLL && cfg.solver_p.solver == XCAL_SOLVER_CG &&
       cfg.solver_p.preconditioner == XCAL_PRECON_DILU) {
-    if (cg_cluster(mixed, P.W, P.n0, ntiles).ctas > 0) form = 1;
+    if (c->cgc.ctas > 0) form = 1;
     else form = ring_tiles(P.W, mixed, c->occ0, ntiles, c->nblocks0) > 0 ? 2 : 3;
   }
   int64_t solvers = cfg.model;
@@ -850,6 +850,14 @@ int xcal_case_setup(xcal_ctx c, const xcal_case *cfg) {
   c->run_cap = 0;
   KParams &h = c->hp;
   int n = c->prep.n;
+  c->cgc = CgCluster{0, 0};
+  c->cg_ctas = 0;
+  if (c->prep.n0 > 0 && c->prep.W <= WUNROLL && cfg->solver_p.solver == XCAL_SOLVER_CG &&
+      cfg->solver_p.preconditioner == XCAL_PRECON_DILU && !(c->flags & XCAL_FLAG_CLUSTER)) {
+    const int mixed = cfg->precision == XCAL_PREC_MIXED;
+    c->cgc = cg_cluster(mixed, c->prep.W, c->prep.n0, h.ntiles);
+    c->cg_ctas = cg_blocks(mixed, c->prep.W, c->device);
+  }
   apply_tuned(c, *cfg);
   DevSink B(c, c->cbuf);
   TRY(case_arrays(c, cfg, B, nullptr, nullptr));
@@ -861,14 +869,6 @@ int xcal_case_setup(xcal_ctx c, const xcal_case *cfg) {
     c->pin = nullptr;
     CUDA_TRY(c, stage_alloc(c, (void **)&c->pin, sizeof(double) * n * 7));
     c->pin_n = (size_t)n * 7;
-  }
-  c->cgc = CgCluster{0, 0};
-  c->cg_ctas = 0;
-  if (h.n0 > 0 && h.AP.W <= WUNROLL && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU &&
-      !(c->flags & XCAL_FLAG_CLUSTER)) {
-    const int mixed = h.prec == XCAL_PREC_MIXED;
-    c->cgc = cg_cluster(mixed, h.AP.W, h.n0, h.ntiles);
-    c->cg_ctas = cg_blocks(mixed, h.AP.W, c->device);
   }
   for (bool &b : c->pin_busy) b = false;
   c->d_stage = c->cbuf.alloc<double>((size_t)n * 7);

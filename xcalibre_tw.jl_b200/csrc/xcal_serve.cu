@@ -159,6 +159,7 @@ struct xcal_server_s {
   bool stop = false;
   int64_t next_ticket = 1;
   xcal_serve_stats st{};
+  int64_t resident = 0;   // cases set up with resident matrix rows
   std::string err;
 };
 
@@ -296,7 +297,7 @@ void setup_main(xcal_server s) {
       s->cv_done.notify_all();
       continue;
     }
-    s->st.resident += j->img.resident;
+    s->resident += j->img.resident;
     s->ready.push_back(j);
     s->cv_sched.notify_all();
   }
@@ -613,6 +614,13 @@ int xcal_serve_stats_get(xcal_server s, xcal_serve_stats *st) {
   st->device_bytes = (double)s->dalloc.cap;
   st->device_bytes_peak = (double)s->dalloc.peak;
   st->grid_ctas = s->grid;
+  return XCAL_OK;
+}
+
+int xcal_serve_resident(xcal_server s, int64_t *cases) {
+  if (!s || !cases) return XCAL_ERR_ARG;
+  std::lock_guard<std::mutex> lk(s->mu);
+  *cases = s->resident;
   return XCAL_OK;
 }
 

@@ -130,7 +130,7 @@ class ServeStats(C.Structure):
     _fields_ = [("submitted", C.c_int64), ("completed", C.c_int64), ("failed", C.c_int64),
                 ("queued", C.c_int64), ("running", C.c_int64), ("cell_iterations", C.c_double),
                 ("run_ms", C.c_double), ("device_bytes", C.c_double), ("device_bytes_peak", C.c_double),
-                ("grid_ctas", C.c_int64), ("resident", C.c_int64)]
+                ("grid_ctas", C.c_int64)]
 
 
 def dptr(a):
@@ -200,6 +200,7 @@ SIGNATURES = {
     "xcal_serve_poll": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32, C.POINTER(ServeResult), P_d,
                                   P_d]),
     "xcal_serve_stats_get": (C.c_int, [C.c_void_p, C.POINTER(ServeStats)]),
+    "xcal_serve_resident": (C.c_int, [C.c_void_p, P_i64]),
     "xcal_serve_destroy": (C.c_int, [C.c_void_p]),
 }
 

@@ -632,7 +632,9 @@ class Server:
     def stats(self):
         st = _abi.ServeStats()
         _abi.check(self.lib.xcal_serve_stats_get(self.srv, C.byref(st)), None, "xcal_serve_stats_get")
-        return {k: getattr(st, k) for k, _ in _abi.ServeStats._fields_}
+        resident = C.c_int64()
+        _abi.check(self.lib.xcal_serve_resident(self.srv, C.byref(resident)), None, "xcal_serve_resident")
+        return dict({k: getattr(st, k) for k, _ in _abi.ServeStats._fields_}, resident=resident.value)
 
     def close(self):
         if getattr(self, "srv", None):
