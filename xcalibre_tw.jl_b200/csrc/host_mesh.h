@@ -42,9 +42,11 @@ void apply_perm(const HostMesh &in, const std::vector<int64_t> &perm, bool reord
 // levels of more than SWEEP_WIDTH rows on average, or any level of more than
 // SWEEP_WIDEST (64 rounds of the CTA's 256 threads, about 0.1 ms: the other CTAs
 // wait meanwhile, and their wait is limited).
-// (ms per SIMPLE iteration, grid / one CTA, by average rows per level: BFS 5k
-// 17: 188 / 117; cavity 40^2 20: 19 / 12; cavity 80^2 40: 84 / 70; hex 12^3 51:
-// 6.0 / 4.5; cavity 160^2 80: 172 / 211; hex 20^3 138: 9.7 / 14.6.)
+// (ms per SIMPLE iteration, grid / one CTA, by average rows per level: BFS 5k 16:
+// 185 / 104; cavity 80^2 40: 65.7 / 36.3; BFS 47k 49: 599 / 532; hex 12^3 51: 4.9 /
+// 3.3; cavity 110^2 55: 106 / 85.7; 120^2 60: 99.8 / 64.7; hex 14^3 69: 4.06 / 3.82;
+// cavity 160^2 80: 166 / 118; hex 16^3 89: 4.65 / 5.93; 20^3 138: 7.49 / 9.17.  In 2D
+// one CTA is still faster somewhat above the line.)
 constexpr int SWEEP_WIDTH = 56, SWEEP_WIDEST = 16384;
 struct LevelLists {
   std::vector<int> frow, brow, items, ptr;

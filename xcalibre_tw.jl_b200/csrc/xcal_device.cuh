@@ -1,7 +1,8 @@
 // Device side of libxcal: data layout, barriers, canonical reductions and the
 // per-row routines of one SIMPLE/PISO iteration.  Everything runs inside one
-// persistent kernel (xcal_kernel.cu); phases are separated by a grid-wide
-// barrier (or a cluster / block barrier for small meshes).
+// persistent kernel (xcal_kernel.cu), or that and a kernel of the pressure CG;
+// phases are separated by a grid-wide barrier (or a cluster / block barrier for
+// small meshes).
 //
 // Arithmetic order: every floating-point expression reproduces the operation
 // order of the reference function it implements (cited per routine), and the
@@ -81,16 +82,17 @@ using Mat = MatT<double>;
 // Most levels that one CTA sweeps while the others wait at a barrier.  A wait
 // is limited (2 s unless the caller sets less), so the work inside one must not
 // grow with the mesh: 1024 levels of at most SWEEP_WIDEST rows (host_mesh.h),
-// about 1.2 ms for levels of a few dozen rows.  The barrier costs about 2 us.
+// about 1 ms for levels of a few dozen rows.  The barrier costs about 2 us.
 constexpr int SWEEP_WAIT = 1024;
 
 // CG in one cluster (xcal_cg_cluster_kernel): most threads of a CTA, vectors,
 // most tiles of the mesh (one partial per lane of the final sum) and of a CTA.
-// At 8 tiles a CTA makes two rounds of a phase; with more the resident form in
-// the program is as fast or faster (ms per SIMPLE iteration, cluster / program:
-// cavity 128^2 0.757 / 1.034, 164^2 0.982 / 1.059, 164^2 mixed 0.912 / 1.063,
-// 200^2 mixed, 10 tiles, 1.160 / 1.084; hex 28^3 0.705 / 0.778, 35^3 mixed, 11
-// tiles, 0.731 / 0.770).
+// At 8 tiles a CTA makes two rounds of a phase, and the resident form in the
+// program is as fast (ms per SIMPLE iteration, cluster / program, with the tiles
+// of the largest share: cavity 64^2, 2, 0.526 / 0.665; 128^2, 4, 0.749 / 0.963;
+// 150^2, 6, 0.837 / 0.972; mixed 164^2, 8, 0.874 / 0.963, 181^2, 8, 0.953 / 0.973;
+// hex 20^3, 2, 0.396 / 0.464; 25^3, 4, 0.875 / 0.965; mixed 30^3, 8, 0.491 /
+// 0.503, 32^3, 8, 0.538 / 0.529).
 constexpr int CGC_TPB = 1024, CGC_VECTORS = 8, CGC_TILES = 256, CGC_SLOTS = 8;
 // Tiles of a group (count N) given to CTA b of G: [chunk(b), chunk(b+1)).
 __host__ __device__ inline int chunk(int b, int N, int G) { return (int)((long long)b * N / G); }

@@ -1,5 +1,7 @@
 // The persistent device program of libxcal: one launch runs `iters` SIMPLE (or
-// PISO) iterations, or one standalone Krylov solve.  Phases are separated by
+// PISO) iterations, or one standalone Krylov solve; or, where the pressure CG is
+// a kernel of its own (small meshes in one cluster, large ones on the whole
+// GPU), what lies between two pressure solves.  Phases are separated by
 // xcal::Sync barriers; every phase is "tile owned" (tile t of 256 rows is always
 // processed by CTA t mod the CTA count), so a CTA may reduce over its tiles at
 // the end of a phase sequence without another barrier.  Reference functions are
@@ -240,11 +242,11 @@ __device__ __forceinline__ void tile_phase(Ctx &C, bool reduce, F f) {
   }
 }
 
-// Rows per thread in the CG phases.  The phases are memory-latency bound (a
-// row is a chain of dependent loads: columns, then neighbour values), so a
-// thread keeps the loads of two rows in flight; the per-row arithmetic is
-// that of the one-row routines.  128^3 cavity: FP64 22.6 -> 21.2 ms per
-// SIMPLE iteration with two rows (preconditioner phases 62 -> 56 us).
+// Rows per thread in the phases of the general CG (any but that over a two-level
+// numbering): the loads of two rows in flight, the arithmetic of the one-row
+// routines.  ms per SIMPLE iteration, two rows / one: 128^3 Jacobi 14.2 / 14.6,
+// mixed 11.8 / 11.3; 96^3 ILU(0) 8.02 / 8.10, DILU in the RCM order 209 / 193,
+// mixed 167 / 136; 800^2 quads, Jacobi, 4.20 / 3.82.
 template <typename T>
 struct CgRows {
   static constexpr int R = 2;
@@ -2433,8 +2435,9 @@ struct Simple {
   }
 };
 
-// The chain of a run.  step < 0: all of it.  Otherwise one link, for large
-// meshes, whose pressure solve is a kernel of its own (xcal_cg_kernel): launch
+// The chain of a run.  step < 0: all of it.  Otherwise one link, for
+// meshes whose pressure solve is a kernel of its own (xcal_cg_kernel,
+// xcal_cg_cluster_kernel): launch
 // `step` does what follows solve step-1 and what leads to solve `step`, and
 // P.step carries the solve's results and the state of the run between them.
 template <int NS, typename T, bool ONE>
@@ -2572,9 +2575,11 @@ __global__ void __launch_bounds__(TPB, MB) xcal_cg_kernel(const __grid_constant_
 //
 // A CTA holds a chunk of the tiles with level-0 rows and the same chunk of
 // the others: its rows are close together in the mesh, so most neighbours
-// are its own, and all CTAs work in each phase.  Up to four tiles at a time,
-// one per 256 threads (threads for tiles that are not there slow the barriers
-// down: cavity 40^2 A 2.57 -> 2.28 us, B and C 1.64 -> 1.54).
+// are its own, and a CTA that has tiles has work in each phase.  (Both splits
+// round alike, so shares differ by up to two tiles: of 16 tiles on 16 CTAs,
+// eight CTAs hold two and eight none.)  Up to four tiles at a time, one per 256
+// threads (threads for tiles that are not there slow the barriers down: cavity
+// 40^2 A 2.57 -> 2.28 us, B and C 1.64 -> 1.54).
 enum { CV_Z = 0, CV_P = 1, CV_R = 3, CV_Q = 5, CV_D = 6, CV_X = 7 };   // vectors (p and r twice)
 static_assert(CV_X + 1 == CGC_VECTORS, "vectors of a row");
 
