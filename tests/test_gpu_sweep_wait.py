@@ -62,3 +62,53 @@ def test_sweep_longer_than_the_wait_limit(precon, monkeypatch):
     xo, ito, _ = O.linear_solve(_abi.SOLVER_CG, precon, rp, col, val, b, np.zeros(n), itmax=2, atol=0.0, rtol=1e-10)
     assert it == ito
     assert np.array_equal(x, xo)
+
+
+def _band(n, h):
+    """Symmetric band of half width h: every row a level, rows of 2h + 1 entries."""
+    rng = np.random.default_rng(h)
+    off = {d: -rng.random(n - d) for d in range(1, h + 1)}
+    rows, cols, vals = [np.arange(n)], [np.arange(n)], [np.full(n, 2.0 * h + 1.0)]
+    for d, v in off.items():
+        i = np.arange(n - d)
+        rows += [i, i + d]
+        cols += [i + d, i]
+        vals += [v, v]
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    o = np.lexsort((c, r))
+    return (np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32), c[o].astype(np.int32), v[o],
+            rng.standard_normal(n))
+
+
+@pytest.mark.parametrize("precon", [_abi.PRECON_DILU, _abi.PRECON_ILU0], ids=["dilu", "ilu0"])
+@pytest.mark.parametrize("n,h", [(700, 3), (700, 4), (1500, 20), (300, 130)])
+def test_wide_rows_match_oracle(precon, n, h):
+    """Rows of 7 (unrolled), 9, 41 and 261 entries: a wait has 1024, 809, 38 and 1 of their levels."""
+    rp, col, val, b = _band(n, h)
+    x, it = _solve(_abi.SOLVER_CG, precon, rp, col, val, b, 4)
+    xo, ito, _ = O.linear_solve(_abi.SOLVER_CG, precon, rp, col, val, b, np.zeros(n), itmax=4, atol=0.0, rtol=1e-10)
+    assert it == ito
+    assert np.array_equal(x, xo)
+
+
+def test_wide_rows_within_the_wait_limit(monkeypatch):
+    """The set-up of ILU(0) takes about 41^2/2 dependent steps of 0.25 us a level:
+    200 ms for 1024 levels, twice the limit here, and 8 ms for the 38 of a wait."""
+    monkeypatch.setenv("XCAL_BARRIER_TIMEOUT_US", "100000")
+    test_wide_rows_match_oracle(_abi.PRECON_ILU0, 1500, 20)
+
+
+@pytest.mark.parametrize("isolated", [16000, 16383, 16384])
+def test_one_wide_level(isolated):
+    """A chain and rows without neighbours: 1500 levels, the first of up to and above the 16,384 rows one CTA sweeps."""
+    rp, col, val, b = _chain(1500)
+    n = 1500 + isolated
+    rp = np.concatenate([rp, rp[-1] + np.arange(1, isolated + 1)]).astype(np.int32)
+    col = np.concatenate([col, np.arange(1500, n)]).astype(np.int32)
+    val = np.concatenate([val, np.full(isolated, 3.0)])
+    b = np.random.default_rng(1).standard_normal(n)
+    x, it = _solve(_abi.SOLVER_CG, _abi.PRECON_DILU, rp, col, val, b, 6)
+    xo, ito, _ = O.linear_solve(_abi.SOLVER_CG, _abi.PRECON_DILU, rp, col, val, b, np.zeros(n), itmax=6, atol=0.0,
+                                rtol=1e-10)
+    assert it == ito
+    assert np.array_equal(x, xo)

@@ -1902,8 +1902,8 @@ int build_case_image(const xcal_mesh_desc *mesh, int renumber, const xcal_case *
   h.conv = tolerance;
   h.abort_nan = 1;
   h.mode = SYNC_GRID;
-  // rows of the case's own group: 40 tiles on 10 CTAs hold 4 each
-  if (h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU)
+  // rows of the case's own group (40 tiles on 10 CTAs: 4 each), by the build that has the CG over two levels
+  if (renumber == XCAL_RENUMBER_COLOR && h.n0 > 0 && h.kP.solver == SOLVER_CG && h.AP.precon == PRECON_DILU)
     h.ring = ring_tiles(h.AU.W, h.prec == XCAL_PREC_MIXED, 1, h.ntiles, c.nblocks);
   if (program_shared_bytes(h.prec == XCAL_PREC_MIXED, h) > group.shared_bytes) h.ring = 0;
   // the server's build has sweeps by one CTA unless it colours (xcal_serve_create)

@@ -83,7 +83,13 @@ using Mat = MatT<double>;
 // is limited (2 s unless the caller sets less), so the work inside one must not
 // grow with the mesh: 1024 levels of at most SWEEP_WIDEST rows (host_mesh.h),
 // about 1 ms for levels of a few dozen rows.  The barrier costs about 2 us.
+// Rows wider than the unrolled ones take longer, up to the square of their width
+// in the set-up of ILU(0), and a wait has fewer of their levels.
 constexpr int SWEEP_WAIT = 1024;
+__device__ __forceinline__ int sweep_wait(int W) {
+  const long long w = W, u = WUNROLL;
+  return w <= u ? SWEEP_WAIT : (int)(w * w >= SWEEP_WAIT * u * u ? 1 : SWEEP_WAIT * u * u / (w * w));
+}
 
 // CG in one cluster (xcal_cg_cluster_kernel): most threads of a CTA, vectors,
 // most tiles of the mesh (one partial per lane of the final sum) and of a CTA.

@@ -374,7 +374,7 @@ __device__ __forceinline__ bool precon_local(const PT &P, const MatT<T> &A, int 
 // solution is no part of, while the other warps pass the levels between, and
 // then works on the vector, which is in shared memory where it fits, when the
 // block barrier of the level before is passed.  The other CTAs wait at a
-// barrier, at most SWEEP_WAIT levels long.  Row arithmetic is that of the row
+// barrier, at most sweep_wait() levels long.  Row arithmetic is that of the row
 // routines.
 // (A count of the items done, polled by the warps, in place of the block
 // barrier: its release waits for the fetches in flight, 1.4 us per level.)
@@ -563,11 +563,11 @@ __device__ __forceinline__ bool precon_tail(Ctx &C, const MatT<T> &A, const T *i
   bool applied = nph == 0 && setup;   // nothing left to apply: reduce in a phase of its own
   if constexpr (ONE) {
     if (C.sweep >= 0 && leveled(A)) {
-      const int levels = sweep_length(C.nfl, C.nbl, first_lvl);
-      for (int lo = 0; lo < levels; lo += SWEEP_WAIT) {
+      const int levels = sweep_length(C.nfl, C.nbl, first_lvl), step = sweep_wait(A.W);
+      for (int lo = 0; lo < levels; lo += step) {
         if (vbid() == 0)
           sweep_by_one<NS, T>(SweepArgs{C.n, C.nfl, C.nbl, C.sweep, C.blev, C.frow, C.brow, C.items, C.lptr}, A, in,
-                              out, setup, first_lvl, lo, min(levels, lo + SWEEP_WAIT));
+                              out, setup, first_lvl, lo, min(levels, lo + step));
         if (!C.sync()) return false;
       }
       applied = true;
