@@ -40,7 +40,8 @@ class _Run:
 
 @pytest.mark.parametrize("geom,n,prec,renumber,kw,form", [
     ("quad", 2, 0, 2, {}, "cluster"), ("quad", 40, 0, 2, {}, "cluster"), ("quad", 155, 1, 2, {}, "cluster"),
-    ("hex", 20, 0, 2, {}, "cluster"), ("hex", 28, 0, 2, {}, "resident"), ("quad", 160, 0, 2, {}, "resident"), ("quad", 200, 1, 2, {}, "resident"),
+    ("hex", 20, 0, 2, {}, "cluster"), ("hex", 28, 0, 2, {}, "resident"),
+    ("quad", 160, 0, 2, {}, "resident"), ("quad", 200, 1, 2, {}, "resident"),
     ("bfs", 27, 0, 2, {}, "resident"), ("hex", 32, 0, 2, {}, "resident"), ("hex", 70, 0, 2, {}, "kernel"),
     ("quad", 40, 0, 0, {}, "general"), ("quad", 40, 0, 2, {"precon": X.Jacobi}, "general"),
     ("quad", 40, 0, 2, {"p_solver": X.BicgstabSolver}, "general")])
